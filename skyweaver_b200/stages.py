@@ -61,6 +61,13 @@ def channel_frequencies(centre, bandwidth, nchans):
 
 
 # ------------------------------------------------------------------ layouts
+def _rows(F, P, A, nsamples, row_stride, device):
+    """FPACT rows for a call that writes `nsamples` of each row: cleared only
+    when that leaves some of a row unwritten."""
+    make = torch.empty if row_stride == nsamples else torch.zeros
+    return make((F, P, A, 2, row_stride), dtype=torch.int8, device=device)
+
+
 def transpose_ftpa(taftp: torch.Tensor, out_nant: int, stream=None) -> torch.Tensor:
     """Transposer::transpose: TAFTP [H][A_in][F][256][2][2] -> FTPA."""
     H, A_in, F = taftp.shape[:3]
@@ -74,7 +81,7 @@ def transpose_fpact(taftp, out_nant, row_stride=None, offset=0, out=None, stream
     T = H * 256
     row_stride = row_stride or (offset + T)
     if out is None:
-        out = torch.zeros((F, 2, out_nant, 2, row_stride), dtype=torch.int8, device=taftp.device)
+        out = _rows(F, 2, out_nant, T, row_stride, taftp.device)
     call("sw_transpose_fpact", _ptr(taftp), _ptr(out), H, A_in, out_nant, F, row_stride,
          offset, _stream(stream))
     return out
@@ -83,7 +90,7 @@ def transpose_fpact(taftp, out_nant, row_stride=None, offset=0, out=None, stream
 def ftpa_to_fpact(ftpa, row_stride=None, offset=0, stream=None):
     F, T, P, A, _ = ftpa.shape
     row_stride = row_stride or (offset + T)
-    out = torch.zeros((F, P, A, 2, row_stride), dtype=torch.int8, device=ftpa.device)
+    out = _rows(F, P, A, T, row_stride, ftpa.device)
     call("sw_ftpa_to_fpact", _ptr(ftpa), _ptr(out), F, T, A, row_stride, offset,
          _stream(stream))
     return out
@@ -118,7 +125,7 @@ def transpose_fpact_statistics(taftp, out_nant, row_stride=None, offset=0, out=N
     T = H * 256
     row_stride = row_stride or (offset + T)
     if out is None:
-        out = torch.zeros((F, 2, out_nant, 2, row_stride), dtype=torch.int8, device=taftp.device)
+        out = _rows(F, 2, out_nant, T, row_stride, taftp.device)
     scratch = torch.empty(lib().sw_statistics_scratch_bytes(F, 2, out_nant), dtype=torch.uint8,
                           device=taftp.device)
     stats = torch.empty((F, 2, out_nant, 4), dtype=torch.float32, device=taftp.device)
