@@ -228,7 +228,7 @@ typedef struct sw_cb_shape {
     int ib_subtract;    /* SKYWEAVER_IB_SUBTRACTION (default 1)           */
     size_t row_stride;  /* FPACT row stride (samples)                     */
     size_t sample_offset;
-    int tiles_per_item; /* 64-sample tiles per work item (0: 64; see sw_autotune) */
+    int tiles_per_item; /* 64-sample tiles per work item (0: 1..64 by the launch's size) */
     int voltage_stages; /* voltage tiles in flight, 2..8 (0: 4; see sw_autotune) */
     int weight_stages;  /* weight blocks in flight, 2..3 (0: 2)                  */
 } sw_cb_shape;

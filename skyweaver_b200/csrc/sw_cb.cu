@@ -46,7 +46,8 @@ constexpr int kN           = 2 * kTileT;
 // per shape by sw_autotune.
 constexpr int kVStagesDefault = 4, kVStagesMax = 8;
 constexpr int kWStagesDefault = 2, kWStagesMax = 3;
-constexpr int kTilesPerItem = 64;  // default work item: 4096 samples of one channel
+constexpr int kMaxTilesPerItem = 64;  // default work item: at most 4096 samples of one channel
+constexpr int kItemCost = 2;  // tiles that an item's start costs (weights, empty pipeline)
 constexpr int kMaxDm       = 16;
 constexpr int kMaxProblems = 96;
 // Epilogue warps: two groups of 8, one per accumulator buffer, so that each
@@ -129,6 +130,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
         : "=r"(ok)
         : "r"(bar), "r"(parity)
         : "memory");
+    return ok != 0;
+}
+
+// One lane of a converged warp, as the compiler can tell: inside
+// `if(elect_one())` the MMA and copy descriptors are known to be uniform and
+// each tcgen05.mma is one instruction.  Under `if(lane == 0)` the same source
+// issues them through a per-lane loop: an issue-only loop of 8 N = 128 MMAs and
+// a commit took 748 cycles that way and 513 elected (512 is the int8 rate).
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok));
     return ok != 0;
 }
 
@@ -359,6 +376,38 @@ __device__ __forceinline__ void stokes_iquv(const uint32_t* r0, const uint32_t* 
     }
 }
 
+// clamp(rint(x / scale)) of the reference, bit for bit, without a division in
+// the usual case.  q = x * r with r = 1 / scale lies within 2^-22.4 |q| of the
+// correctly rounded quotient, that is within 2.4e-5 where q is inside the
+// clamp, so both round to the same integer unless q is that close to a
+// half-integer; only those values (about 1 in 10^4) are divided.  A scale whose
+// reciprocal is not an ordinary number divides every value (limit < 0).
+// Clamping first gives the same result, and adding 1.5 * 2^23 leaves the
+// rounded integer in the low byte.  FAST is taken where a column group of 16
+// samples has two outputs or more; with one the branch costs more than it
+// saves (benchmark's 4 DMs on 16 channels, divided / FAST: tscrunch 4 4.92 /
+// 4.42 ms, 8 2.71 / 2.50 ms, 16 2.14 / 2.27 ms).
+template <bool FAST>
+struct Quant {
+    float scale, r, limit;
+    __device__ __forceinline__ explicit Quant(float s) : scale(s)
+    {
+        r = __frcp_rn(s);
+        const float a = fabsf(s);
+        limit = a > 1e-30f && a < 1e30f ? 0.5f - 3.0517578125e-5f : -1.0f;
+    }
+    __device__ __forceinline__ uint32_t operator()(float x) const
+    {
+        const float kMagic = 12582912.0f;
+        auto clamped = [](float v) { return fmaxf(-128.0f, fminf(127.0f, v)); };
+        if constexpr(!FAST) return __float_as_uint(fadd(clamped(fdiv(x, scale)), kMagic)) & 0xffu;
+        const float c = clamped(fmul(x, r));
+        float m = fadd(c, kMagic);
+        if(fabsf(fsub(c, fsub(m, kMagic))) > limit) m = fadd(clamped(fdiv(x, scale)), kMagic);
+        return __float_as_uint(m) & 0xffu;
+    }
+};
+
 struct Item {
     int p, f, tc, b0;
 };
@@ -436,7 +485,7 @@ cb_kernel(const __grid_constant__ Params P)
     const int ntiles_gulp = P.nsamples / kTileT;
 
     if(warp == 0) {
-        if(lane == 0 && !P.test_stall) {
+        if(elect_one() && !P.test_stall) {
             // ---------------------------------------------------- producer
             const uint32_t wbuf_s = smem_u32(wbuf), vbuf_s = smem_u32(vbuf);
             int vs = 0, ws = 0;
@@ -483,7 +532,7 @@ cb_kernel(const __grid_constant__ Params P)
             }
         }
     } else if(warp == 1) {
-        if(lane == 0) {
+        if(elect_one()) {
             // ------------------------------------------------- MMA issuer
             // This thread shares its SM sub-partition with four busy
             // epilogue warps, so its per-tile instruction count bounds how
@@ -545,12 +594,6 @@ cb_kernel(const __grid_constant__ Params P)
         // group leave too few registers for it
         constexpr int kG      = (STOKES == 4 && TS <= 4) ? 8 : 16;
         constexpr int kGroups = kSlice / kG;         // column groups per warp
-        // Release the accumulator buffer as soon as the tile's last column
-        // group is in registers, before its arithmetic, when several outputs
-        // per group follow the last load (tscrunch <= 8: measured 3.4 %
-        // faster at tscrunch 8); at tscrunch 16 the release after the
-        // arithmetic measured 0.9 % faster.
-        constexpr bool kEarlyRelease = TS <= 8;
         const int q   = warp & 3;               // TMEM lane quarter of this warp
         const int h   = ((warp - 2) >> 2) % kHalves;  // which part of the tile's samples
         const int grp = (warp - 2) / (kEpiWarps / 2); // accumulator buffer this warp drains
@@ -570,7 +613,7 @@ cb_kernel(const __grid_constant__ Params P)
             const int b = it.b0 + q * 32 + lane;
             const bool valid = (b < pr.beam_start + pr.beam_count) && (b < P.nbeams);
             const int bs = valid ? P.mapping[b] : 0;
-            const float scale = P.scale[bs * F + it.f];
+            const Quant<(STOKES == 4 ? 4 : 1) * 16 / TS >= 2> quant(P.scale[bs * F + it.f]);
             const float offs  = P.offset[bs * F + it.f];
             const int tile0 = it.tc * P.tpi;
             const int tile1 = min(ntiles_gulp, tile0 + P.tpi);
@@ -635,7 +678,10 @@ cb_kernel(const __grid_constant__ Params P)
                         SW_TMEM_LD8(ta + 192, i1);
                     }
                     tmem_wait_ld();
-                    if(kEarlyRelease && g == kGroups - 1) {
+                    if(g == kGroups - 1) {
+                        // all of the tile is in registers: the next tile's MMAs
+                        // run behind this group's arithmetic (release after it
+                        // instead: 2.40 against 2.11 ms at tscrunch 16)
                         fence_before();
                         __syncwarp();
                         if(lane == 0) mbar_arrive(&acc_empty[grp]);
@@ -663,47 +709,37 @@ cb_kernel(const __grid_constant__ Params P)
                         if(emit) {
                             const int e = u / TS;  // emit index within the slice
                             if constexpr(NC == 1) {
-                                float v;
+                                float v = power[0];
                                 if(P.ib_subtract) {
                                     const float ib = kPrefetch ? ibp[kPrefetch ? e : 0] : ibq[e * ib_emit];
-                                    v = rintf(fdiv(fsub(power[0], fmul(ib, 16129.0f)), scale));
+                                    v = fsub(v, fmul(ib, 16129.0f));
                                 } else if(STOKES == 0) {
-                                    v = rintf(fdiv(fsub(power[0], offs), scale));
-                                } else {
-                                    v = rintf(fdiv(power[0], scale));
+                                    v = fsub(v, offs);
                                 }
-                                if(valid) outp[e * out_emit] = clamp_i8(v);
+                                const uint32_t o = quant(v);
+                                if(valid) outp[e * out_emit] = (int8_t)o;
                             } else {
                                 // char4 {I, Q, U, V}; the IB power is float4
-                                float v[4];
+                                float v[4] = {power[0], power[1], power[2], power[3]};
                                 if(P.ib_subtract) {
                                     const float4 ib = kPrefetch
                                         ? make_float4(ibp[0], ibp[1], ibp[2], ibp[3])
                                         : reinterpret_cast<const float4*>(ibq)[e * F];
-                                    v[0] = rintf(fdiv(fsub(power[0], fmul(ib.x, 16129.0f)), scale));
-                                    v[1] = rintf(fdiv(fsub(power[1], fmul(ib.y, 16129.0f)), scale));
-                                    v[2] = rintf(fdiv(fsub(power[2], fmul(ib.z, 16129.0f)), scale));
-                                    v[3] = rintf(fdiv(fsub(power[3], fmul(ib.w, 16129.0f)), scale));
+                                    v[0] = fsub(v[0], fmul(ib.x, 16129.0f));
+                                    v[1] = fsub(v[1], fmul(ib.y, 16129.0f));
+                                    v[2] = fsub(v[2], fmul(ib.z, 16129.0f));
+                                    v[3] = fsub(v[3], fmul(ib.w, 16129.0f));
                                 } else {
-                                    v[0] = rintf(fdiv(fsub(power[0], offs), scale));
-                                    v[1] = rintf(fdiv(power[1], scale));
-                                    v[2] = rintf(fdiv(power[2], scale));
-                                    v[3] = rintf(fdiv(power[3], scale));
+                                    v[0] = fsub(v[0], offs);
                                 }
-                                if(valid)
-                                    reinterpret_cast<char4*>(outp)[e * F * P.nbeams] =
-                                        make_char4(clamp_i8(v[0]), clamp_i8(v[1]),
-                                                   clamp_i8(v[2]), clamp_i8(v[3]));
+                                const uint32_t o = quant(v[0]) | quant(v[1]) << 8 |
+                                                   quant(v[2]) << 16 | quant(v[3]) << 24;
+                                if(valid) reinterpret_cast<uint32_t*>(outp)[e * F * P.nbeams] = o;
                             }
 #pragma unroll
                             for(int c = 0; c < NC; ++c) power[c] = 0.0f;
                         }
                     }
-                }
-                if(!kEarlyRelease) {
-                    fence_before();
-                    __syncwarp();
-                    if(lane == 0) mbar_arrive(&acc_empty[grp]);
                 }
                 aph ^= 1;
                 outp += (2 * kTileT / TS) * out_emit;
@@ -810,6 +846,29 @@ int num_sms()
     return n;
 }
 
+// Default work-item size in tiles for `blocks` (128-beam block, channel) pairs
+// of `tiles` tiles each: the CTA with the most items works through
+// cdiv(items, SMs) of them, each costing its tiles plus kItemCost, and the
+// size that makes this least is taken (the larger of equals).  Large launches
+// get the longest items (64 tiles: 128 measured 2-6 % slower at tscrunch 16
+// and 4), small ones enough items for every SM: 64 beams x 8 channels x 4096
+// samples ran as 8 items of 64 tiles on 8 SMs in 92 us and run as 128 items of
+// 4 tiles in 12 us.
+int default_tiles_per_item(long blocks, int tiles)
+{
+    int best = 1;
+    long least = 0;
+    for(int n = 1; n <= kMaxTilesPerItem; ++n) {
+        const long items = blocks * cdiv(tiles, n);
+        const long cost = cdiv(items, (long)num_sms()) * ((n < tiles ? n : tiles) + kItemCost);
+        if(n == 1 || cost <= least) {
+            least = cost;
+            best = n;
+        }
+    }
+    return best;
+}
+
 int launch(const sw_cb_shape* s, const sw_cb_problem* probs, int nprob,
            const void* w, const float* scale, const float* offset,
            const int* mapping, int32_t* debug, cudaStream_t stream,
@@ -843,7 +902,11 @@ int launch(const sw_cb_shape* s, const sw_cb_problem* probs, int nprob,
     int ndm = 0, item = 0;
     SW_REQUIRE(s->tiles_per_item >= 0 && s->tiles_per_item <= 1024,
                "CoherentBeamformer: tiles_per_item must be in [0, 1024]");
-    const int tpi = s->tiles_per_item > 0 ? s->tiles_per_item : kTilesPerItem;
+    long blocks = 0;
+    for(int i = 0; i < nprob; ++i)
+        if(probs[i].beam_count > 0) blocks += (long)s->nchans * cdiv(probs[i].beam_count, kM);
+    const int tpi = s->tiles_per_item > 0 ? s->tiles_per_item
+                                          : default_tiles_per_item(blocks, s->nsamples / kTileT);
     const int ntc = cdiv(s->nsamples / kTileT, tpi);
     for(int i = 0; i < nprob; ++i) {
         const sw_cb_problem& pr = probs[i];
