@@ -30,6 +30,7 @@
 // memory; FFT arithmetic is FP32.
 #include <algorithm>
 
+#include "sw_cdd_pk.cuh"
 #include "sw_common.cuh"
 
 namespace swb {
@@ -327,7 +328,7 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p)
 // otherwise with plain byte copies.
 template <int N, int NT>
 __device__ __forceinline__ void stage_input(uint8_t* st, const Args& A, int item, int L,
-                                            bool aligned)
+                                            bool aligned, int tid)
 {
     const int stream = item / A.nseg;
     const int seg    = item - stream * A.nseg;
@@ -337,7 +338,7 @@ __device__ __forceinline__ void stage_input(uint8_t* st, const Args& A, int item
     const int avail = A.overlap + A.nsamples;
     if(aligned) {
         constexpr int kChunks = N / 16;
-        for(int c = threadIdx.x; c < 2 * kChunks; c += NT) {
+        for(int c = tid; c < 2 * kChunks; c += NT) {
             const int plane = c >= kChunks;
             const int k     = (c - plane * kChunks) * 16;
             const int left  = avail - (start + k);
@@ -350,7 +351,7 @@ __device__ __forceinline__ void stage_input(uint8_t* st, const Args& A, int item
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     } else {
-        for(int i = threadIdx.x; i < N; i += NT) {
+        for(int i = tid; i < N; i += NT) {
             const int idx = start + i;
             st[i]     = idx < avail ? row_re[idx] : 0;
             st[N + i] = idx < avail ? row_im[idx] : 0;
@@ -358,10 +359,43 @@ __device__ __forceinline__ void stage_input(uint8_t* st, const Args& A, int item
     }
 }
 
-// at least two resident CTAs per SM below N = 8192 (latency hiding across
-// the per-pass barriers); N = 8192 needs 512 threads and fits one.
+// The DMs of exactly 0 (bits of zero_dms): their output is the staged window
+// itself, trimmed like the others.
+template <int N, int NT>
+__device__ __forceinline__ void copy_zero_dms(const uint8_t* stage, const Args& A,
+                                              uint32_t zero_dms, int stream, int start, int L,
+                                              int head, bool copy16, int tid)
+{
+    for(uint32_t zm = zero_dms; zm; zm &= zm - 1) {
+        const int d = __ffs(zm) - 1;
+        uint8_t* o_re = A.out[d] + (size_t)stream * 2 * A.out_stride;
+        const int n = min(L, A.nsamples - start);  // kept samples of this window
+        if(copy16 && ((reinterpret_cast<uintptr_t>(A.out[d]) & 15) == 0)) {
+            const int chunks = (n + 15) / 16;
+            for(int c = tid; c < 2 * chunks; c += NT) {
+                const int plane = c >= chunks;
+                const int k = (c - plane * chunks) * 16;
+                const uint8_t* src = stage + plane * N + head + k;
+                uint8_t* dst = o_re + plane * A.out_stride + start + k;
+                if(k + 16 <= n) {
+                    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+                } else {
+                    for(int b = 0; b < n - k; ++b) dst[b] = src[b];
+                }
+            }
+        } else {
+            for(int i = tid; i < 2 * n; i += NT) {
+                const int plane = i >= n, k = i - plane * n;
+                o_re[plane * A.out_stride + start + k] = stage[plane * N + head + k];
+            }
+        }
+    }
+}
+
+// Windows of 256 and 512 points, one per CTA of 16 points a thread; several
+// CTAs per SM hide the latency across the per-pass barriers.
 template <int LOGN, bool DBG>
-__global__ void __launch_bounds__((1 << LOGN) / 16, LOGN >= 13 ? 1 : (LOGN == 12 ? 2 : 4))
+__global__ void __launch_bounds__((1 << LOGN) / 16, 4)
 cdd_kernel(const __grid_constant__ Args A)
 {
     constexpr int N  = 1 << LOGN;
@@ -389,7 +423,7 @@ cdd_kernel(const __grid_constant__ Args A)
     if constexpr(!DBG)
         for(int d = 0; d < A.ndms && d < 32; ++d) zero_dms |= (A.zero_flags[d] ? 1u : 0u) << d;
     const bool copy16 = aligned && (head % 16) == 0 && (A.out_stride % 16) == 0;
-    if(blockIdx.x < nitems) stage_input<N, NT>(stage, A, blockIdx.x, L, aligned);
+    if(blockIdx.x < nitems) stage_input<N, NT>(stage, A, blockIdx.x, L, aligned, threadIdx.x);
     for(int item = blockIdx.x; item < nitems; item += gridDim.x) {
         const int stream = item / A.nseg;
         const int seg    = item - stream * A.nseg;
@@ -421,35 +455,12 @@ cdd_kernel(const __grid_constant__ Args A)
                 for(int q = 0; q < R0; ++q) buf[pad_at(j, pad(j), q, s0)] = x[q];
             }
         }
-        for(uint32_t zm = zero_dms; zm; zm &= zm - 1) {
-            const int d = __ffs(zm) - 1;
-            uint8_t* o_re = A.out[d] + (size_t)stream * 2 * A.out_stride;
-            const int n = min(L, A.nsamples - start);  // kept samples of this window
-            if(copy16 && ((reinterpret_cast<uintptr_t>(A.out[d]) & 15) == 0)) {
-                const int chunks = (n + 15) / 16;
-                for(int c = threadIdx.x; c < 2 * chunks; c += NT) {
-                    const int plane = c >= chunks;
-                    const int k = (c - plane * chunks) * 16;
-                    const uint8_t* src = stage + plane * N + head + k;
-                    uint8_t* dst = o_re + plane * A.out_stride + start + k;
-                    if(k + 16 <= n) {
-                        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-                    } else {
-                        for(int b = 0; b < n - k; ++b) dst[b] = src[b];
-                    }
-                }
-            } else {
-                for(int i = threadIdx.x; i < 2 * n; i += NT) {
-                    const int plane = i >= n, k = i - plane * n;
-                    o_re[plane * A.out_stride + start + k] = stage[plane * N + head + k];
-                }
-            }
-        }
+        copy_zero_dms<N, NT>(stage, A, zero_dms, stream, start, L, head, copy16, threadIdx.x);
         __syncthreads();
         // the staging buffer is free: fetch the next work item's window now so
         // that its global-memory latency hides behind this item's transforms
         if(item + (int)gridDim.x < nitems)
-            stage_input<N, NT>(stage, A, item + gridDim.x, L, aligned);
+            stage_input<N, NT>(stage, A, item + gridDim.x, L, aligned, threadIdx.x);
         // ---- forward radix-16 passes except the last
 #pragma unroll
         for(int p = 1; p < P.npass - 1; ++p) {
@@ -535,6 +546,123 @@ cdd_kernel(const __grid_constant__ Args A)
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// Windows of 1024 .. 8192 points: 16384 / N windows per CTA, each by a group of
+// N / 32 threads with its own barrier and staging buffer (sw_cdd_pk.cuh).
+//
+// One window per CTA at 16 points a thread (scalar arithmetic, one more pass,
+// twiddles in shared memory, spectrum in registers: cdd_kernel) was bound by
+// shared-memory wavefronts (63 %), issue (61 %) and its CTA-wide barriers:
+// 64 antennas x 64 channels x 65536 samples at DMs 50, 150 and 500 took 9.21 ms
+// that way with 8192 points and take 5.50 ms here; 32 channels x 32768 samples
+// with 4096 points 2.10 -> 1.33 ms; 48 antennas x 32 channels x 16384 samples,
+// one DM, with 2048 points 0.285 -> 0.207 ms.  With 16 warps of 126 registers per
+// SM no unit is saturated: FMA pipe and shared-memory wavefronts 54 %, issue
+// 48 %.  (Barriers for the whole group after every pass: 5.81 ms.)
+template <int LOGN, bool DBG>
+__global__ void __launch_bounds__(kPkThreads, 1)
+cdd_pk_kernel(const __grid_constant__ Args A)
+{
+    using G = PkGeo<LOGN>;
+    constexpr int N = G::N, NT = G::T;
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ uint32_t s_tmem;
+    PkGroup g;
+    const uint32_t tmem = pk_setup<LOGN>(g, smem, &s_tmem, reinterpret_cast<const float*>(A.tw));
+    const int t = g.t;
+    uint8_t* stage = smem + kPkBufBytes + g.window * 2 * N;
+
+    const int L = N - A.overlap;
+    const int head = A.overlap - A.lag;  // trimmed at the start of each window
+    const float inv_n = 1.0f / (float)N;  // exact (power of two)
+    const int nitems = A.nstreams * A.nseg;
+    const bool aligned = (A.row_stride % 16 == 0) && (L % 16 == 0) &&
+                         ((reinterpret_cast<uintptr_t>(A.in) & 15) == 0);
+    // DMs of exactly 0: copied from the staged window (see cdd_kernel)
+    uint32_t zero_dms = 0;
+    if constexpr(!DBG)
+        for(int d = 0; d < A.ndms && d < 32; ++d) zero_dms |= (A.zero_flags[d] ? 1u : 0u) << d;
+    const bool copy16 = aligned && (head % 16) == 0 && (A.out_stride % 16) == 0;
+    // both samples of a pair are kept or trimmed together and their bytes may
+    // be stored as one 16-bit word
+    const bool even = ((head | L | A.nsamples) & 1) == 0 && (A.out_stride & 1) == 0;
+    // v / N rounded to the nearest even integer in the low mantissa bits (v / N
+    // is below 2^14 in magnitude): the low byte is the int8-wrapped sample
+    const uint64_t scale = pk2(inv_n, inv_n), magic = pk2(12582912.0f, 12582912.0f);
+    const int step = G::W * gridDim.x;
+    int item = g.window * gridDim.x + blockIdx.x;
+    if(item < nitems) stage_input<N, NT>(stage, A, item, L, aligned, t);
+    for(; item < nitems; item += step) {
+        const int stream = item / A.nseg;
+        const int seg    = item - stream * A.nseg;
+        const int f      = stream / A.npa;
+        const int start  = seg * L;  // first input sample of the window
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        pk_sync<LOGN>(g);
+        copy_zero_dms<N, NT>(stage, A, zero_dms, stream, start, L, head, copy16, t);
+        Pk x[16];
+#pragma unroll
+        for(int r = 0; r < 16; ++r) {
+            const uint32_t re = *reinterpret_cast<const uint16_t*>(stage + 2 * t + (N / 16) * r);
+            const uint32_t im = *reinterpret_cast<const uint16_t*>(stage + N + 2 * t + (N / 16) * r);
+            x[r] = {pk2((float)(int8_t)re, (float)(int8_t)(re >> 8)),
+                    pk2((float)(int8_t)im, (float)(int8_t)(im >> 8))};
+        }
+        // the next window's bytes are fetched behind this one's transforms
+        pk_forward<LOGN>(g, x, [&] {
+            if(item + step < nitems)
+                stage_input<N, NT>(stage, A, item + step, L, aligned, t);
+        });
+        const float4* chp = reinterpret_cast<const float4*>(A.chirp + (size_t)f * N) + t;
+        // samples of this window that the output holds: window index head + u,
+        // output sample start + u, u < kept
+        const unsigned kept = (unsigned)max(0, min(L, A.nsamples - start));
+        const size_t out_at = (size_t)stream * 2 * A.out_stride + start;
+        for(int d = 0; d < A.ndms; ++d) {
+            if(d < 32 && ((zero_dms >> d) & 1u)) continue;
+            pk_inverse<LOGN>(g, chp + (size_t)d * A.chirp_dm_stride / 2, x);
+            uint8_t* o_re = A.out[d] + out_at;
+            uint8_t* o_im = o_re + A.out_stride;
+            const bool words = even && (reinterpret_cast<uintptr_t>(A.out[d]) & 1) == 0;
+#pragma unroll
+            for(int r = 0; r < 16; ++r) {
+                const int u = 2 * t + (N / 16) * r - head;
+                uint32_t ra, rb, ia, ib;
+                unpk2u(pfma(x[r].re, scale, magic), ra, rb);
+                unpk2u(pfma(x[r].im, scale, magic), ia, ib);
+                if(words) {
+                    if((unsigned)u < kept) {
+                        *reinterpret_cast<uint16_t*>(o_re + u) =
+                            (uint16_t)__byte_perm(ra, rb, 0x0040);
+                        *reinterpret_cast<uint16_t*>(o_im + u) =
+                            (uint16_t)__byte_perm(ia, ib, 0x0040);
+                    }
+                } else {
+                    if((unsigned)u < kept) {
+                        o_re[u] = (uint8_t)ra;
+                        o_im[u] = (uint8_t)ia;
+                    }
+                    if((unsigned)(u + 1) < kept) {
+                        o_re[u + 1] = (uint8_t)rb;
+                        o_im[u + 1] = (uint8_t)ib;
+                    }
+                }
+                if constexpr(DBG) {
+                    float fr[2], fi[2];
+                    unpk2(pmul(x[r].re, scale), fr[0], fr[1]);
+                    unpk2(pmul(x[r].im, scale), fi[0], fi[1]);
+                    for(int e = 0; e < 2; ++e)
+                        if((unsigned)(u + e) < kept)
+                            A.dbg[((size_t)d * A.nstreams + stream) * A.nsamples + start + u + e] =
+                                make_float2(fr[e], fi[e]);
+                }
+            }
+            pk_sync<LOGN>(g);  // the next store of this group waits for these loads
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    pk_tmem_free(tmem);
+}
+
 // ------------------------------------------------- long FFTs (N = S x 8192)
 // Overlap-save windows longer than one CTA's shared memory are split four-step
 // style into S = N / 8192 sub-transforms of M = 8192 points:
@@ -543,11 +671,15 @@ cdd_kernel(const __grid_constant__ Args A)
 //                 W_N^(n2 k1) * sum_n1 x[M n1 + n2] W_S^(n1 k1)
 //   inverse:  x[n2 + M n1] = sum_k1 W_S^(-n1 k1) *
 //                 W_N^(-n2 k1) * IDFT_M over k2 of Y[k1 + S k2]
-// cdd_split_kernel runs one (segment, k1) per CTA: the S-point partial DFT
-// straight from the int8 rows, the M-point forward FFT, and for every DM the
-// chirp of bins k1 + S k2 and the M-point inverse FFT, leaving
-// W_N^(-n2 k1) * z in a complex workspace; cdd_split_combine then does the
-// S-point inverse DFT over k1, the overlap-save trim, /N, rint and int8 wrap.
+// cdd_split_kernel runs one (segment, k1) per group of 256 threads: the S-point
+// partial DFT straight from the int8 rows into pass 0's registers, the M-point
+// forward FFT, and for every DM the chirp of bins k1 + S k2 and the M-point
+// inverse FFT (sw_cdd_pk.cuh), leaving W_N^(-n2 k1) * z in a workspace of pairs
+// (8-byte accesses: the caller's workspace need not be aligned further); cdd_split_combine then does the S-point inverse DFT over k1,
+// the overlap-save trim, /N, rint and int8 wrap.  DMs of exactly 0 are copied
+// from the rows by the combine step.
+// 64 antennas x 8 channels x 65536 samples at 65536 points and DMs 0, 50, 150
+// and 500: 7.46 ms with 16 points a thread in scalar arithmetic, 4.12 ms so.
 constexpr int kSplitLog = 13;
 constexpr int kSplitM   = 1 << kSplitLog;
 
@@ -559,8 +691,9 @@ struct SplitArgs {
     int item0, nitems;  // work items [item0, item0 + nitems) of this chunk
     const c32* tw;      // M-point plan tables
     const c32* chirp;   // [ndms][F][S][M]: bin k1 + S k2 at k1's per-thread load order
-    const c32* tws;     // [S][M]: W_N^(n2 k1)
-    c32* z;             // [ndms][nitems][S][M]
+    const float4* tws;  // [S][M / 2] pair quads: W_N^(n2 k1)
+    float2* z;          // [ndms][nitems][S][re|im][M / 2] pairs
+    const uint32_t* zero_flags;  // [ndms]: non-zero if the DM is 0 (chirp exactly 1)
     uint8_t* out[kMaxDms];
     size_t out_stride;
     float2* dbg;
@@ -584,106 +717,91 @@ __device__ __forceinline__ c32 wsm(int m)
 }
 
 template <int S>
-__global__ void __launch_bounds__(kSplitM / 16, 1)
+__global__ void __launch_bounds__(kPkThreads, 1)
 cdd_split_kernel(const __grid_constant__ SplitArgs A)
 {
-    constexpr int LOGN = kSplitLog;
-    constexpr int M  = kSplitM;
-    constexpr int N  = S * M;
-    constexpr int NT = M / 16;
-    constexpr Plan P = make_plan(LOGN);
-    constexpr int R0 = P.r0;
-    constexpr int B0 = 16 / R0;
+    constexpr int LOGN = kSplitLog, M = kSplitM, N = S * M;
+    using G = PkGeo<LOGN>;
     extern __shared__ __align__(16) uint8_t smem[];
-    c32* buf  = reinterpret_cast<c32*>(smem);
-    c32* tw_s = buf + pad(M) + 16;
-    for(int i = threadIdx.x; i < P.tw_total; i += NT) tw_s[i] = A.tw[i];
+    __shared__ uint32_t s_tmem;
+    PkGroup g;
+    const uint32_t tmem = pk_setup<LOGN>(g, smem, &s_tmem, reinterpret_cast<const float*>(A.tw));
+    const int t = g.t;
     const int L = N - A.overlap;
     const int avail = A.overlap + A.nsamples;
+    const bool even = ((L | (int)(A.row_stride & 1)) & 1) == 0 &&
+                      (reinterpret_cast<uintptr_t>(A.in) & 1) == 0;
 
-    for(int u = blockIdx.x; u < A.nitems * S; u += gridDim.x) {
+    const int nunits = A.nitems * S;
+    for(int u = g.window * gridDim.x + blockIdx.x; u < nunits; u += G::W * gridDim.x) {
         const int il = u / S, k1 = u - il * S;
         const int item   = A.item0 + il;
         const int stream = item / A.nseg;
         const int seg    = item - stream * A.nseg;
         const int f      = stream / A.npa;
         const int start  = seg * L;
-        const int8_t* row_re = reinterpret_cast<const int8_t*>(A.in) + (size_t)stream * 2 * A.row_stride;
-        const int8_t* row_im = row_re + A.row_stride;
-        __syncthreads();  // previous unit's last reads of buf are done
-        // ---- S-point partial DFT for this k1, times W_N^(n2 k1)
-#pragma unroll 4
-        for(int v = 0; v < 16; ++v) {
-            const int n2 = threadIdx.x + v * NT;
-            c32 acc{0.0f, 0.0f};
+        const uint8_t* row_re = A.in + (size_t)stream * 2 * A.row_stride + start + 2 * t;
+        const uint8_t* row_im = row_re + A.row_stride;
+        // ---- S-point partial DFT for this k1, times W_N^(n2 k1), n2 = 2 t + 512 r
+        Pk x[16];
 #pragma unroll
-            for(int n1 = 0; n1 < S; ++n1) {
-                const int idx = start + n1 * M + n2;
-                const c32 x = idx < avail ? c32{(float)row_re[idx], (float)row_im[idx]}
-                                          : c32{0.0f, 0.0f};
-                acc = cadd(acc, cmul(x, wsm<S>(n1 * k1)));
+        for(int r = 0; r < 16; ++r) x[r] = {0, 0};
+#pragma unroll 1
+        for(int n1 = 0; n1 < S; ++n1) {
+            const c32 w = wsm<S>(n1 * k1);
+            const Pk wp = {pk2(w.x, w.x), pk2(w.y, w.y)};
+            const int left = avail - (start + n1 * M + 2 * t);  // samples from this thread's first
+            if(avail - (start + n1 * M) <= 0) break;            // zero padding from here on
+#pragma unroll
+            for(int r = 0; r < 16; ++r) {
+                const int at = n1 * M + 512 * r;
+                uint32_t re = 0, im = 0;
+                if(even && 512 * r + 1 < left) {
+                    re = *reinterpret_cast<const uint16_t*>(row_re + at);
+                    im = *reinterpret_cast<const uint16_t*>(row_im + at);
+                } else {
+                    if(512 * r < left) { re = row_re[at]; im = row_im[at]; }
+                    if(512 * r + 1 < left) {
+                        re |= (uint32_t)row_re[at + 1] << 8;
+                        im |= (uint32_t)row_im[at + 1] << 8;
+                    }
+                }
+                const uint64_t xr = pk2((float)(int8_t)re, (float)(int8_t)(re >> 8));
+                const uint64_t xi = pk2((float)(int8_t)im, (float)(int8_t)(im >> 8));
+                x[r].re = psub(pfma(xr, wp.re, x[r].re), pmul(xi, wp.im));
+                x[r].im = pfma(xi, wp.re, pfma(xr, wp.im, x[r].im));
             }
-            buf[pad(n2)] = cmul(acc, A.tws[(size_t)k1 * M + n2]);
         }
-        __syncthreads();
-        // ---- M-point forward FFT (DIF) in shared memory
-        fwd_pass<LOGN, R0>(buf, tw_s, P.span[0], P.stride[0], P.tw_off[0]);
-        __syncthreads();
+        const float4* tws = A.tws + (size_t)k1 * (M / 2) + t;
+        if(k1 > 0) {
 #pragma unroll
-        for(int p = 1; p < P.npass - 1; ++p) {
-            fwd_pass<LOGN, 16>(buf, tw_s, P.span[p], P.stride[p], P.tw_off[p]);
-            __syncthreads();
+            for(int r = 0; r < 16; ++r) {
+                const float4 w = tws[256 * r];
+                x[r] = pcmul<false>(x[r], Pk{pk2(w.x, w.y), pk2(w.z, w.w)});
+            }
         }
-        c32 spec[16];
-#pragma unroll
-        for(int r = 0; r < 16; ++r) spec[r] = buf[pad(threadIdx.x * 16 + r)];
-        dft16<false>(spec);
-        const size_t chirp_dm = A.chirp_dm_stride;  // complex per DM
-        const float4* chp = reinterpret_cast<const float4*>(A.chirp + (size_t)f * N + (size_t)k1 * M) + threadIdx.x;
-        __syncthreads();
+        pk_sync<LOGN>(g);  // the previous unit's last reads of shared memory are done
+        pk_forward<LOGN>(g, x, [] {});
+        const float4* chp =
+            reinterpret_cast<const float4*>(A.chirp + (size_t)f * N + (size_t)k1 * M) + t;
         for(int d = 0; d < A.ndms; ++d) {
-            const float4* cd = chp + (size_t)d * chirp_dm / 2;
-            c32 y[16];
+            if(A.zero_flags[d] && !A.dbg) continue;
+            pk_inverse<LOGN>(g, chp + (size_t)d * A.chirp_dm_stride / 2, x);
+            float2* zo = A.z + (((size_t)d * A.nitems + il) * S + k1) * M + t;
 #pragma unroll
-            for(int k = 0; k < 8; ++k) {
-                const float4 c = cd[k * NT];
-                y[2 * k]     = cmul(spec[2 * k], c32{c.x, c.y});
-                y[2 * k + 1] = cmul(spec[2 * k + 1], c32{c.z, c.w});
+            for(int r = 0; r < 16; ++r) {
+                const float4 w = tws[256 * r];
+                const Pk z = pcmul<true>(x[r], Pk{pk2(w.x, w.y), pk2(w.z, w.w)});
+                float2 re, im;
+                unpk2(z.re, re.x, re.y);
+                unpk2(z.im, im.x, im.y);
+                zo[256 * r]         = re;
+                zo[M / 2 + 256 * r] = im;
             }
-            dft16<true>(y);
-#pragma unroll
-            for(int r = 0; r < 16; ++r) buf[pad(threadIdx.x * 16 + r)] = y[r];
-            __syncthreads();
-#pragma unroll
-            for(int p = P.npass - 2; p >= 1; --p) {
-                inv_pass<LOGN, 16>(buf, tw_s, P.span[p], P.stride[p], P.tw_off[p]);
-                __syncthreads();
-            }
-            // last inverse pass, then W_N^(-n2 k1), to the workspace
-            c32* zo = A.z + (((size_t)d * A.nitems + il) * S + k1) * M;
-            constexpr int s0 = M / R0;
-#pragma unroll
-            for(int v = 0; v < B0; ++v) {
-                const int j = threadIdx.x + v * NT;
-                c32 z[R0];
-#pragma unroll
-                for(int q = 0; q < R0; ++q) z[q] = buf[pad_at(j, pad(j), q, s0)];
-                {
-                    c32 w[R0];
-                    load_tw<R0>(tw_s, P.tw_off[0], s0, j, w);
-#pragma unroll
-                    for(int q = 1; q < R0; ++q) z[q] = cmulc(z[q], w[q]);
-                }
-                dft<R0, true>(z);
-#pragma unroll
-                for(int r = 0; r < R0; ++r) {
-                    const int n2 = j + r * s0;
-                    zo[n2] = cmulc(z[r], A.tws[(size_t)k1 * M + n2]);
-                }
-            }
-            __syncthreads();
+            pk_sync<LOGN>(g);
         }
     }
+    pk_tmem_free(tmem);
 }
 
 template <int S>
@@ -693,35 +811,60 @@ cdd_split_combine(const __grid_constant__ SplitArgs A)
     constexpr int M = kSplitM, N = S * M;
     const int L = N - A.overlap, head = A.overlap - A.lag;
     const float inv_n = 1.0f / (float)N;  // exact (power of two)
-    const size_t total = (size_t)A.ndms * A.nitems * M;
+    // as in cdd_pk_kernel: the low byte of v / N + 1.5 2^23 is the sample
+    const uint64_t scale = pk2(inv_n, inv_n), magic = pk2(12582912.0f, 12582912.0f);
+    const size_t total = (size_t)A.ndms * A.nitems * (M / 2);
     for(size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
         idx += (size_t)gridDim.x * blockDim.x) {
-        const int n2 = (int)(idx % M);
-        const size_t rest = idx / M;
+        const int n2 = 2 * (int)(idx % (M / 2));
+        const size_t rest = idx / (M / 2);
         const int il = (int)(rest % A.nitems);
         const int d  = (int)(rest / A.nitems);
         const int item   = A.item0 + il;
         const int stream = item / A.nseg;
         const int seg    = item - stream * A.nseg;
         const int start  = seg * L;
-        const c32* zi = A.z + ((size_t)d * A.nitems + il) * S * M + n2;
-        c32 z[S];
-#pragma unroll
-        for(int k1 = 0; k1 < S; ++k1) z[k1] = zi[(size_t)k1 * M];
-        dft<S, true>(z);  // z[n1] = sum_k1 W_S^(-n1 k1) z'[k1]
-        uint8_t* o_re = A.out[d] + (size_t)stream * 2 * A.out_stride;
+        const unsigned kept = (unsigned)max(0, min(L, A.nsamples - start));
+        uint8_t* o_re = A.out[d] + (size_t)stream * 2 * A.out_stride + start;
         uint8_t* o_im = o_re + A.out_stride;
+        if(A.zero_flags[d] && !A.dbg) {
+            const uint8_t* i_re = A.in + (size_t)stream * 2 * A.row_stride + start + head;
+            for(int n1 = 0; n1 < S; ++n1)
+                for(int e = 0; e < 2; ++e) {
+                    const int v = n2 + e + n1 * M - head;
+                    if((unsigned)v < kept) {
+                        o_re[v] = i_re[v];
+                        o_im[v] = i_re[A.row_stride + v];
+                    }
+                }
+            continue;
+        }
+        const float2* zi = A.z + ((size_t)d * A.nitems + il) * S * M + n2 / 2;
+        Pk z[S];
+#pragma unroll
+        for(int k1 = 0; k1 < S; ++k1) {
+            const float2 re = zi[(size_t)k1 * M], im = zi[(size_t)k1 * M + M / 2];
+            z[k1] = {pk2(re.x, re.y), pk2(im.x, im.y)};
+        }
+        pdft<S, true>(z);  // z[n1] = sum_k1 W_S^(-n1 k1) z'[k1]
 #pragma unroll
         for(int n1 = 0; n1 < S; ++n1) {
-            const int i = n2 + n1 * M;
-            const int m = start + i - head;
-            if(i >= head && i < head + L && m < A.nsamples) {
-                const float fr = z[n1].x * inv_n, fi = z[n1].y * inv_n;
-                o_re[m] = (uint8_t)__float2int_rn(fr);
-                o_im[m] = (uint8_t)__float2int_rn(fi);
-                if(A.dbg)
-                    A.dbg[((size_t)d * A.nstreams + stream) * A.nsamples + m] = make_float2(fr, fi);
-            }
+            const int v = n2 + n1 * M - head;
+            uint32_t re[2], im[2];
+            unpk2u(pfma(z[n1].re, scale, magic), re[0], re[1]);
+            unpk2u(pfma(z[n1].im, scale, magic), im[0], im[1]);
+            float fr[2], fi[2];
+            unpk2(pmul(z[n1].re, scale), fr[0], fr[1]);
+            unpk2(pmul(z[n1].im, scale), fi[0], fi[1]);
+#pragma unroll
+            for(int e = 0; e < 2; ++e)
+                if((unsigned)(v + e) < kept) {
+                    o_re[v + e] = (uint8_t)re[e];
+                    o_im[v + e] = (uint8_t)im[e];
+                    if(A.dbg)
+                        A.dbg[((size_t)d * A.nstreams + stream) * A.nsamples + start + v + e] =
+                            make_float2(fr[e], fi[e]);
+                }
         }
     }
 }
@@ -729,8 +872,7 @@ cdd_split_combine(const __grid_constant__ SplitArgs A)
 template <int S>
 int launch_split(SplitArgs a, int total_items, size_t ws_items, cudaStream_t stream)
 {
-    constexpr Plan P = make_plan(kSplitLog);
-    const size_t smem = (size_t)(pad(kSplitM) + 16 + ((P.tw_total + 1) & ~1)) * sizeof(c32);
+    const size_t smem = kPkBufBytes;
     SW_CUDA_CHECK(cudaFuncSetAttribute(cdd_split_kernel<S>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int dev = 0, nsm = 148;
@@ -740,9 +882,9 @@ int launch_split(SplitArgs a, int total_items, size_t ws_items, cudaStream_t str
         a.item0  = i0;
         a.nitems = (int)std::min<size_t>(ws_items, (size_t)(total_items - i0));
         const long units = (long)a.nitems * S;
-        cdd_split_kernel<S><<<(int)std::min<long>(units, nsm), kSplitM / 16, smem, stream>>>(a);
+        cdd_split_kernel<S><<<(int)std::min<long>(units, nsm), kPkThreads, smem, stream>>>(a);
         SW_LAUNCH_CHECK();
-        const size_t total = (size_t)a.ndms * a.nitems * kSplitM;
+        const size_t total = (size_t)a.ndms * a.nitems * (kSplitM / 2);
         const size_t blocks = std::min<size_t>(cdiv(total, (size_t)256), (size_t)nsm * 16);
         cdd_split_combine<S><<<(int)blocks, 256, 0, stream>>>(a);
         SW_LAUNCH_CHECK();
@@ -788,6 +930,46 @@ __global__ void twiddle_k(c32* tw, int logn)
     }
 }
 
+// Twiddles of the packed transform (PkGeo: pass 0's quads, then pass 1's).
+__global__ void twiddle_pk_k(float4* tw, int logn)
+{
+    const int n = 1 << logn, cols0 = n / 32, cols1 = n / 512;
+    for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < 15 * (cols0 + cols1);
+        i += gridDim.x * blockDim.x) {
+        const bool first = i < 15 * cols0;
+        const int k = first ? i : i - 15 * cols0, cols = first ? cols0 : cols1;
+        const int q = 1 + k / cols, j = 2 * (k % cols), span = first ? n : n / 16;
+        double s0, c0, s1, c1;
+        sincospi(-2.0 * (double)(j * q) / (double)span, &s0, &c0);
+        sincospi(-2.0 * (double)((j + 1) * q) / (double)span, &s1, &c1);
+        tw[i] = make_float4((float)c0, (float)c1, (float)s0, (float)s1);
+    }
+}
+template <int LOGN>
+constexpr bool pk_twiddles_fit()
+{
+    return (PkGeo<LOGN>::TW0 + PkGeo<LOGN>::TW1) * 2 <= make_plan(LOGN).tw_total;
+}
+static_assert(pk_twiddles_fit<10>() && pk_twiddles_fit<11>() && pk_twiddles_fit<12>() &&
+                  pk_twiddles_fit<13>(),
+              "setup block layout");
+
+// Entry q of an N-point chirp table in the packed transform's order: quad
+// (i, t) at i * (N / 32) + t holds the two bins of pair i of thread t as
+// (re, re, im, im).
+struct PkBin {
+    int bin;
+    int word;  // of the table: the real part; the imaginary part is 2 words on
+};
+__device__ __forceinline__ PkBin pk_bin(int logn, int q)
+{
+    const int n = 1 << logn, r2 = n / 256, cols = n / 32;
+    const int h = q & 1, quad = q >> 1, t = quad % cols, i = quad / cols;
+    const int block = t * (32 / r2) + i / (r2 / 2);  // transform of pass 2
+    const int k = i % (r2 / 2) + h * (r2 / 2);
+    return {block / 16 + 16 * (block % 16) + 256 * k, 4 * quad + h};
+}
+
 // DMResponse (CoherentDedisperser.cu:313-335) in FP64.  The transform
 // leaves bin digit_reverse(16 t + r) in register r of thread t; the table
 // stores the chirp of that bin at ((r / 2) * (N / 16) + t) * 2 + r % 2, so
@@ -805,13 +987,23 @@ __global__ void chirp_k(c32* chirp, SetupArgs S)
         const int d   = (int)(i / ((size_t)P.n * S.nchans));
         const int t   = (q >> 1) % nt;
         const int r   = 2 * ((q >> 1) / nt) + (q & 1);
-        const int k   = digit_reverse(P, 16 * t + r);
+        const bool pk = S.logn >= kPkMinLog;
+        const PkBin b = pk ? pk_bin(S.logn, q) : PkBin{};
+        const int k   = pk ? b.bin : digit_reverse(P, 16 * t + r);
         const double nu0   = S.low_freq + c * S.coarse_bw - 0.5 * S.coarse_bw;
         const double nu    = k * S.fine_bw;
         const double phase = (nu * nu * S.prefactor[d]) / ((nu0 + nu) * nu0 * nu0);
         double sn, cs;
         sincos(phase, &sn, &cs);
-        chirp[i] = c32{(float)cs, (float)sn};
+        if(pk) {
+            // a chirp that is no number (a DM that is none) gives zeros
+            const bool ok = isfinite(cs) && isfinite(sn);
+            float* w = reinterpret_cast<float*>(chirp + (i - q)) + b.word;
+            w[0] = ok ? (float)cs : 0.0f;
+            w[2] = ok ? (float)sn : 0.0f;
+        } else {
+            chirp[i] = c32{(float)cs, (float)sn};
+        }
     }
 }
 
@@ -819,8 +1011,6 @@ __global__ void chirp_k(c32* chirp, SetupArgs S)
 // at k1 * M + (the M-point per-thread load order of k2).
 __global__ void chirp_split_k(c32* chirp, SetupArgs S, int split)
 {
-    const Plan P = make_plan(kSplitLog);
-    const int nt = kSplitM / 16;
     const int n  = split * kSplitM;
     const size_t total = (size_t)S.ndms * S.nchans * n;
     for(size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
@@ -829,27 +1019,31 @@ __global__ void chirp_split_k(c32* chirp, SetupArgs S, int split)
         const int c  = (int)((i / n) % S.nchans);
         const int d  = (int)(i / ((size_t)n * S.nchans));
         const int k1 = q / kSplitM, qq = q % kSplitM;
-        const int t  = (qq >> 1) % nt;
-        const int r  = 2 * ((qq >> 1) / nt) + (qq & 1);
-        const int k  = k1 + split * digit_reverse(P, 16 * t + r);
+        const PkBin b = pk_bin(kSplitLog, qq);
+        const int k  = k1 + split * b.bin;
         const double nu0   = S.low_freq + c * S.coarse_bw - 0.5 * S.coarse_bw;
         const double nu    = k * S.fine_bw;
         const double phase = (nu * nu * S.prefactor[d]) / ((nu0 + nu) * nu0 * nu0);
         double sn, cs;
         sincos(phase, &sn, &cs);
-        chirp[i] = c32{(float)cs, (float)sn};
+        const bool ok = isfinite(cs) && isfinite(sn);
+        float* w = reinterpret_cast<float*>(chirp + (i - qq)) + b.word;
+        w[0] = ok ? (float)cs : 0.0f;
+        w[2] = ok ? (float)sn : 0.0f;
     }
 }
 
-// W_N^(n2 k1) = exp(-2 pi i n2 k1 / N) in FP64, [k1][n2]
-__global__ void split_twiddle_k(c32* tws, int split)
+// W_N^(n2 k1) = exp(-2 pi i n2 k1 / N) in FP64, [k1][n2 / 2] pair quads
+__global__ void split_twiddle_k(float* tws, int split)
 {
     const int n = split * kSplitM;
     for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int k1 = i / kSplitM, n2 = i % kSplitM;
         double sn, cs;
         sincospi(-2.0 * (double)((long long)n2 * k1) / (double)n, &sn, &cs);
-        tws[i] = c32{(float)cs, (float)sn};
+        float* w = tws + 4 * (i / 2) + (i & 1);  // n2 = i mod M: pairs stay together
+        w[0] = (float)cs;
+        w[2] = (float)sn;
     }
 }
 
@@ -872,6 +1066,28 @@ int launch_logn_dbg(const Args& a, cudaStream_t stream)
     cdd_kernel<LOGN, DBG><<<(int)grid, N / 16, smem, stream>>>(a);
     SW_LAUNCH_CHECK();
     return SW_OK;
+}
+
+template <int LOGN, bool DBG>
+int launch_pk_dbg(const Args& a, cudaStream_t stream)
+{
+    const size_t smem = kPkBufBytes + kPkStageBytes;
+    SW_CUDA_CHECK(cudaFuncSetAttribute(cdd_pk_kernel<LOGN, DBG>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    // the first window of every SM before the second of any
+    const long items = (long)a.nstreams * a.nseg;
+    cdd_pk_kernel<LOGN, DBG><<<(int)std::min<long>(items, nsm), kPkThreads, smem, stream>>>(a);
+    SW_LAUNCH_CHECK();
+    return SW_OK;
+}
+
+template <int LOGN>
+int launch_pk(const Args& a, cudaStream_t stream)
+{
+    return a.dbg ? launch_pk_dbg<LOGN, true>(a, stream) : launch_pk_dbg<LOGN, false>(a, stream);
 }
 
 // the float output for precision studies is a separate instance, so the
@@ -943,8 +1159,9 @@ int launch_cdd(const void* d_fpact_in, size_t row_stride, int nchans, int npol, 
         a.chirp_dm_stride = (size_t)setup_nchans * fft_len;
         a.tw = tw;
         a.chirp = ch;
-        a.tws = ch_all + (size_t)setup_ndms * setup_nchans * fft_len;
-        a.z = static_cast<c32*>(d_workspace);
+        a.tws = reinterpret_cast<const float4*>(ch_all + (size_t)setup_ndms * setup_nchans * fft_len);
+        a.z = static_cast<float2*>(d_workspace);
+        a.zero_flags = zero_flags;
         for(int d = 0; d < ndms; ++d) {
             SW_REQUIRE(h_d_out[d], "coherent dedispersion: null output for DM %d", d);
             a.out[d] = static_cast<uint8_t*>(h_d_out[d]);
@@ -982,10 +1199,10 @@ int launch_cdd(const void* d_fpact_in, size_t row_stride, int nchans, int npol, 
     switch(logn) {
     case 8: return launch_logn<8>(a, s);
     case 9: return launch_logn<9>(a, s);
-    case 10: return launch_logn<10>(a, s);
-    case 11: return launch_logn<11>(a, s);
-    case 12: return launch_logn<12>(a, s);
-    default: return launch_logn<13>(a, s);
+    case 10: return launch_pk<10>(a, s);
+    case 11: return launch_pk<11>(a, s);
+    case 12: return launch_pk<12>(a, s);
+    default: return launch_pk<13>(a, s);
     }
 }
 
@@ -1019,7 +1236,9 @@ int sw_cdd_chirps(const float* h_dms, int ndms, int nchans, int fft_len,
     const Plan P = make_plan(plog);
     c32* tw = static_cast<c32*>(d_setup);
     c32* ch = tw + P.tw_total + kSetupGap;
-    twiddle_k<<<64, 256, 0, as_cuda(stream)>>>(tw, plog);
+    if(plog >= kPkMinLog)
+        twiddle_pk_k<<<32, 128, 0, as_cuda(stream)>>>(reinterpret_cast<float4*>(tw), plog);
+    else twiddle_k<<<64, 256, 0, as_cuda(stream)>>>(tw, plog);
     SW_LAUNCH_CHECK();
     // the words after the twiddle tables flag the DMs of exactly 0
     ZeroFlags zf{};
@@ -1040,8 +1259,8 @@ int sw_cdd_chirps(const float* h_dms, int ndms, int nchans, int fft_len,
         const int split = fft_len / kSplitM;
         chirp_split_k<<<148 * 4, 256, 0, as_cuda(stream)>>>(ch, S, split);
         SW_LAUNCH_CHECK();
-        split_twiddle_k<<<64, 256, 0, as_cuda(stream)>>>(ch + (size_t)ndms * nchans * fft_len,
-                                                         split);
+        split_twiddle_k<<<64, 256, 0, as_cuda(stream)>>>(
+            reinterpret_cast<float*>(ch + (size_t)ndms * nchans * fft_len), split);
         SW_LAUNCH_CHECK();
     } else {
         chirp_k<<<148 * 4, 256, 0, as_cuda(stream)>>>(ch, S);

@@ -77,3 +77,61 @@ def test_coherent_beam_default_work_items(cuda, B, F, T):
     out = [_np(stages.coherent_beamform(fp, w, scl, off, mapping, None, T, ts, ib_subtract=False,
                                         tiles_per_item=n)) for n in (0, 1, 1024)]
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("n,F,P,A,T,ov,lag,dms,pad", [
+    (8192, 1, 2, 1, 7000, 1600, 128, [500.0], 0),          # one window
+    (8192, 2, 2, 37, 6593, 1600, 128, [50.0, 500.0], 7),   # odd samples and stride: byte stores
+    (8192, 1, 1, 3, 20000, 1333, 401, [0.0, 333.0], 16),   # odd overlap and lag, odd window count
+    (8192, 3, 2, 50, 16, 48, 16, [3.0, 0.0, 2.0], 0),      # a few samples; more windows than SMs
+    (8192, 2, 2, 4, 40000, 8000, 4000, [150.0], 2),        # 192 useful samples per window
+    (4096, 2, 2, 5, 9001, 1334, 400, [0.0, 100.0, 300.0], 3),
+    (4096, 3, 2, 64, 3000, 96, 16, [20.0], 8),
+    (2048, 3, 2, 33, 5000, 501, 77, [10.0, 0.0], 1),
+    (2048, 1, 1, 1, 64, 32, 16, [1.0], 0),
+    (1024, 2, 2, 21, 10000, 240, 128, [5.0, 30.0], 4),
+    (1024, 1, 2, 7, 2001, 111, 30, [0.0, 7.0], 3),
+    (512, 2, 2, 9, 3000, 97, 20, [3.0], 1),
+    (16384, 1, 2, 3, 20001, 1601, 129, [0.0, 300.0], 3),   # split transforms
+    (32768, 2, 1, 2, 5000, 3000, 128, [0.0, 400.0], 0),
+    (65536, 1, 2, 2, 70000, 1600, 128, [500.0, 0.0, 50.0], 6),
+])
+def test_coherent_dedispersion_windows(cuda, n, F, P, A, T, ov, lag, dms, pad):
+    """Windows of every length at odd trims, strides and window counts against
+    torch's FP64 transform: bytes differ only where the FP64 value lies within
+    the transform's single-precision error of a half-integer, and the float
+    outputs by no more than that.  The error bound is log2 n butterfly stages
+    of 2^-24 each way on values of rms 12 sqrt(2), times 8 for the largest of
+    10^6."""
+    from skyweaver_b200 import stages
+    torch = cuda
+    g = np.random.default_rng(T + ov)
+    chbw = 856e6 / 1024
+    bw, low = F * chbw, 1257e6
+    tol = 8 * 2 * np.log2(n) * 2.0 ** -24 * 17.0
+    ext = np.clip(np.rint(g.normal(0, 12, size=(F, P, A, 2, ov + T + pad))), -127, 127)
+    ext = _dev(cuda, ext.astype(np.int8))
+    cdd = stages.CoherentDedisperser(F, A, n, ov, low, bw, dms, lag=lag)
+    outs = [torch.full((F, P, A, 2, T + pad), 99, dtype=torch.int8, device="cuda") for _ in dms]
+    plain = [o.clone() for o in outs]
+    _, dbg = cdd.dedisperse(ext, T, outs=outs, debug=True)
+    cdd.dedisperse(ext, T, outs=plain)
+    z = torch.complex(ext[..., 0, :ov + T].double(), ext[..., 1, :ov + T].double())
+    step = n - ov
+    for d, dm in enumerate(dms):
+        k = torch.arange(n, dtype=torch.float64, device="cuda") * (chbw / n)
+        nu0 = (low + (torch.arange(F, dtype=torch.float64, device="cuda") - 0.5) * chbw)[:, None]
+        ph = -2 * np.pi * 4.148806423e15 * float(np.float32(dm)) * k * k / ((nu0 + k) * nu0 * nu0)
+        chirp = torch.polar(torch.ones_like(ph), ph)[:, None, None]
+        ref = torch.empty((F, P, A, T), dtype=torch.complex128, device="cuda")
+        for s in range(0, T, step):
+            win = torch.nn.functional.pad(z[..., s:s + n], (0, max(0, s + n - z.shape[-1])))
+            y = torch.fft.ifft(torch.fft.fft(win) * chirp)[..., ov - lag:ov - lag + step]
+            ref[..., s:s + step] = y[..., :T - s]
+        r = torch.stack([ref.real, ref.imag], -2)
+        for o in (outs[d], plain[d]):
+            assert bool((o[..., T:] == 99).all())
+            err = (o[..., :T].double() - r).abs()
+            assert float(err.max()) <= 0.5 + tol, (dm, float(err.max()))
+        f = torch.view_as_complex(dbg[d]).to(torch.complex128)
+        assert float((f - ref).abs().max()) <= tol
