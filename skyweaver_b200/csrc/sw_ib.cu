@@ -225,6 +225,244 @@ ib_k(IbArgs args, int bs0)
     }
 }
 
+// tscrunch 4, 8, 16 and 32 on rows aligned to 16 bytes: every thread takes one
+// 16-byte run of samples (two for 32) of a channel, that is 16 / TS outputs,
+// for a quarter of the antennas; the four warps of a CTA share 32 runs and add
+// their exact integer sums in shared memory.
+//
+// ib_k gives a thread all antennas of one output: 4-byte loads below tscrunch
+// 16, sums of all four Stokes parameters for 8 beamsets in 64 bits whatever is
+// asked for, and too few threads on short gulps.  Here the Stokes parameter
+// and the number of beamsets are compile-time choices and sums stay in 32
+// bits: the bound sum(max |w| I) that decides whether they are exact saturates
+// at 2^29, and a sum can only wrap where that bound is far above 2^24.  Bound
+// by HBM (one read of the voltages).  64 antennas: 8 beamsets on 64 channels x
+// 32768 samples at tscrunch 8 214 -> 115 us (537 MB, 4.7 TB/s), one beamset on
+// 256 channels x 16384 samples 386 -> 163 us (6.6 TB/s); 8 channels x 4096
+// samples of 16 antennas at tscrunch 4 18 -> 5.6 us.
+constexpr int kIbWarps = 4;
+
+// The reference's float chain (t outer, a inner, float multiply and add) of
+// one output, from a table of its products (see ib_k), or sample by sample
+// when the antennas exceed the table.  First decides in 64 bits whether this
+// beamset's own sum is exact after all (`sum` holds it).
+template <int TS>
+__device__ __noinline__ float ib_chain(const IbArgs& args, int f, int t0, const float* w,
+                                       bool int_weights, int stokes, int sum)
+{
+    constexpr int L = TS < 16 ? TS : 16;  // samples per step
+    const size_t rs = args.row_stride;
+    const uint8_t* p0 = args.fpact + ((size_t)f * 2 * args.nant) * 2 * rs + args.offset + t0;
+    const uint8_t* p1 = p0 + (size_t)args.nant * 2 * rs;
+    if(int_weights) {
+        long long bound = 0;
+        for(int a = 0; a < args.nant; ++a) {
+            int e = 0;
+            for(int r = 0; r < 2; ++r)
+                for(int k = 0; k < TS; k += 4) {
+                    const int x = *reinterpret_cast<const int*>(p0 + (2 * a + r) * rs + k);
+                    const int y = *reinterpret_cast<const int*>(p1 + (2 * a + r) * rs + k);
+                    e = __dp4a(x, x, __dp4a(y, y, e));
+                }
+            bound += (long long)fabsf(w[a]) * e;
+        }
+        if(bound <= (1ll << 24)) return (float)sum;
+    }
+    float power = 0.0f;
+    for(int tc = 0; tc < TS; tc += L) {
+        if(args.nant <= kTableAnt) {
+            float x[L][kTableAnt];
+#pragma unroll 2
+            for(int a = 0; a < args.nant; ++a) {
+                uint32_t v[4][L / 4];
+#pragma unroll
+                for(int k = 0; k < L / 4; ++k) {
+                    v[0][k] = *reinterpret_cast<const uint32_t*>(p0 + 2 * a * rs + tc + 4 * k);
+                    v[1][k] = *reinterpret_cast<const uint32_t*>(p0 + (2 * a + 1) * rs + tc + 4 * k);
+                    v[2][k] = *reinterpret_cast<const uint32_t*>(p1 + 2 * a * rs + tc + 4 * k);
+                    v[3][k] = *reinterpret_cast<const uint32_t*>(p1 + (2 * a + 1) * rs + tc + 4 * k);
+                }
+#pragma unroll
+                for(int k = 0; k < L; ++k) {
+                    auto byte = [&](int r) { return (float)(int8_t)(v[r][k / 4] >> (8 * (k & 3))); };
+                    x[k][a] = fmul(stokes_f(stokes, byte(0), byte(1), byte(2), byte(3)), w[a]);
+                }
+            }
+            for(int k = 0; k < L; ++k)
+                for(int a = 0; a < args.nant; ++a) power = fadd(power, x[k][a]);
+        } else {
+            for(int k = tc; k < tc + L; ++k)
+                for(int a = 0; a < args.nant; ++a)
+                    power = fadd(power, fmul(stokes_f(stokes, (float)(int8_t)p0[2 * a * rs + k],
+                                                      (float)(int8_t)p0[(2 * a + 1) * rs + k],
+                                                      (float)(int8_t)p1[2 * a * rs + k],
+                                                      (float)(int8_t)p1[(2 * a + 1) * rs + k]),
+                                             w[a]));
+        }
+    }
+    return power;
+}
+
+// NC components (4: I, Q, U, V), NBS beamsets per pass; I_ONLY: NC = 1 and
+// Stokes I.
+template <int TS, int NC, int NBS, bool I_ONLY>
+__global__ void __launch_bounds__(32 * kIbWarps)
+ib_run_k(const __grid_constant__ IbArgs args, int bs0)
+{
+    constexpr int NO = TS < 16 ? 16 / TS : 1;   // outputs per thread
+    constexpr int RUN = TS < 16 ? 16 : TS;      // samples per thread
+    constexpr int NV = NO * (NBS * NC + 1);     // sums per thread, the bounds last
+    __shared__ float sw[NBS][kMaxAnt];
+    __shared__ int s_max[kMaxAnt];              // max |w| over the beamsets, >= 2^24: not whole
+    __shared__ int s_int[NBS];
+    __shared__ uint32_t red[kIbWarps][NV][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nbs = min(NBS, args.nbeamsets - bs0);
+    if(threadIdx.x < NBS) s_int[threadIdx.x] = 1;
+    __syncthreads();
+    for(int a = threadIdx.x; a < args.nant; a += blockDim.x) {
+        int m = 0;
+#pragma unroll
+        for(int s = 0; s < NBS; ++s) {
+            const float w = s < nbs ? args.weights[(size_t)(bs0 + s) * args.nant + a] : 0.0f;
+            sw[s][a] = w;
+            const bool ok = (w == rintf(w)) && fabsf(w) <= 1024.0f;
+            if(!ok) s_int[s] = 0;
+            else m = max(m, abs((int)w));
+        }
+        s_max[a] = m;
+    }
+    __syncthreads();
+
+    const int f  = args.chan_order ? args.chan_order[blockIdx.y] : (int)blockIdx.y;
+    const int t0 = (blockIdx.x * 32 + lane) * RUN;
+    uint32_t S[NO][NBS * NC], B[NO];
+#pragma unroll
+    for(int o = 0; o < NO; ++o) {
+        B[o] = 0;
+#pragma unroll
+        for(int i = 0; i < NBS * NC; ++i) S[o][i] = 0;
+    }
+    if(t0 < args.nsamples) {
+        const size_t rs = args.row_stride;
+        const uint8_t* p0 = args.fpact + ((size_t)f * 2 * args.nant) * 2 * rs + args.offset + t0;
+        const uint8_t* p1 = p0 + (size_t)args.nant * 2 * rs;
+#pragma unroll 4
+        for(int a = warp; a < args.nant; a += kIbWarps) {
+            uint32_t pI[NO], p[NO][NC];
+#pragma unroll
+            for(int o = 0; o < NO; ++o) {
+                pI[o] = 0;
+#pragma unroll
+                for(int c = 0; c < NC; ++c) p[o][c] = 0;
+            }
+#pragma unroll
+            for(int k = 0; k < RUN; k += 16) {
+                const uint4 R0 = *reinterpret_cast<const uint4*>(p0 + 2 * a * rs + k);
+                const uint4 I0 = *reinterpret_cast<const uint4*>(p0 + (2 * a + 1) * rs + k);
+                const uint4 R1 = *reinterpret_cast<const uint4*>(p1 + 2 * a * rs + k);
+                const uint4 I1 = *reinterpret_cast<const uint4*>(p1 + (2 * a + 1) * rs + k);
+                const int r0[4] = {(int)R0.x, (int)R0.y, (int)R0.z, (int)R0.w};
+                const int i0[4] = {(int)I0.x, (int)I0.y, (int)I0.z, (int)I0.w};
+                const int r1[4] = {(int)R1.x, (int)R1.y, (int)R1.z, (int)R1.w};
+                const int i1[4] = {(int)I1.x, (int)I1.y, (int)I1.z, (int)I1.w};
+#pragma unroll
+                for(int q = 0; q < 4; ++q) {
+                    const int o = NO == 1 ? 0 : q * 4 / TS;
+                    if constexpr(I_ONLY) {
+                        pI[o] = __dp4a(r0[q], r0[q], __dp4a(i0[q], i0[q], __dp4a(r1[q], r1[q],
+                                       __dp4a(i1[q], i1[q], (int)pI[o]))));
+                    } else {
+                        const int e0 = __dp4a(r0[q], r0[q], __dp4a(i0[q], i0[q], 0));
+                        const int e1 = __dp4a(r1[q], r1[q], __dp4a(i1[q], i1[q], 0));
+                        const int u = 2 * __dp4a(r0[q], r1[q], __dp4a(i0[q], i1[q], 0));
+                        const int v = 2 * (__dp4a(i0[q], r1[q], 0) - __dp4a(r0[q], i1[q], 0));
+                        pI[o] += e0 + e1;
+                        if constexpr(NC == 4) {
+                            p[o][0] += e0 + e1;
+                            p[o][1] += e0 - e1;
+                            p[o][2] += u;
+                            p[o][3] += v;
+                        } else {
+                            p[o][0] += args.stokes == 0 ? e0 + e1 : args.stokes == 1 ? e0 - e1
+                                     : args.stokes == 2 ? u : v;
+                        }
+                    }
+                }
+            }
+            const uint32_t m = s_max[a];
+#pragma unroll
+            for(int o = 0; o < NO; ++o) {
+                // |w| I <= 2^10 2^21 per antenna, four warps: no wrap
+                B[o] = min(B[o] + m * pI[o], 1u << 29);
+#pragma unroll
+                for(int s = 0; s < NBS; ++s) {
+                    const uint32_t wi = (uint32_t)(int)sw[s][a];
+#pragma unroll
+                    for(int c = 0; c < NC; ++c)
+                        S[o][s * NC + c] += wi * (I_ONLY ? pI[o] : p[o][c]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for(int o = 0; o < NO; ++o) {
+#pragma unroll
+        for(int i = 0; i < NBS * NC; ++i) red[warp][o * NBS * NC + i][lane] = S[o][i];
+        red[warp][NO * NBS * NC + o][lane] = B[o];
+    }
+    __syncthreads();
+    if(t0 >= args.nsamples) return;
+
+    const int nout = args.nsamples / TS;
+    for(int i = warp; i < NO * nbs; i += kIbWarps) {
+        const int o = i % NO, s = i / NO, bs = bs0 + s;
+        const int tp = t0 / TS + o;
+        uint32_t bound = 0;
+        for(int k = 0; k < kIbWarps; ++k) bound += red[k][NO * NBS * NC + o][lane];
+        const size_t at = ((size_t)bs * nout + tp) * args.nchans + f;
+        const size_t so = (size_t)bs * args.nchans + f;
+        for(int c = 0; c < NC; ++c) {
+            const int stokes = NC == 4 ? c : args.stokes;
+            uint32_t sum = 0;
+            for(int k = 0; k < kIbWarps; ++k) sum += red[k][(o * NBS + s) * NC + c][lane];
+            const float power = s_int[s] && bound <= (1u << 24)
+                                    ? (float)(int)sum  // the float chain is exact
+                                    : ib_chain<TS>(args, f, tp * TS, sw[s], s_int[s] != 0, stokes,
+                                                   (int)sum);
+            args.raw[at * NC + c] = power;
+            const float sc = stokes == 0
+                                 ? rintf(fdiv(fsub(power, args.offset_v[so]), args.scale[so]))
+                                 : rintf(fdiv(power, args.scale[so]));
+            args.out[at * NC + c] = clamp_i8(sc);
+        }
+    }
+}
+
+template <int TS, int NC, int NBS, bool I_ONLY>
+int launch_runs(const IbArgs& args, cudaStream_t stream)
+{
+    const dim3 grid(cdiv(args.nsamples / (TS < 16 ? 16 : TS), 32), args.nchans);
+    for(int bs0 = 0; bs0 < args.nbeamsets; bs0 += NBS) {
+        ib_run_k<TS, NC, NBS, I_ONLY><<<grid, 32 * kIbWarps, 0, stream>>>(args, bs0);
+        SW_LAUNCH_CHECK();
+    }
+    return SW_OK;
+}
+
+template <int TS>
+int launch_ts(const IbArgs& args, cudaStream_t stream)
+{
+    if(args.stokes == 4)
+        return args.nbeamsets == 1 ? launch_runs<TS, 4, 1, false>(args, stream)
+                                   : launch_runs<TS, 4, 2, false>(args, stream);
+    if(args.stokes == 0)
+        return args.nbeamsets == 1 ? launch_runs<TS, 1, 1, true>(args, stream)
+                                   : launch_runs<TS, 1, 8, true>(args, stream);
+    return args.nbeamsets == 1 ? launch_runs<TS, 1, 1, false>(args, stream)
+                               : launch_runs<TS, 1, 8, false>(args, stream);
+}
+
 }  // namespace
 
 int launch_incoherent_beamform(const void* d_fpact, size_t row_stride,
@@ -250,6 +488,16 @@ int launch_incoherent_beamform(const void* d_fpact, size_t row_stride,
     IbArgs args{static_cast<const uint8_t*>(d_fpact), row_stride, sample_offset,
                 nchans, nsamples, nant, tscrunch, nbeamsets, stokes, d_scale,
                 d_offset, d_beamset_weights, d_raw, d_out, d_chan_order};
+    // whole aligned 16-byte runs of samples per thread
+    if(nsamples % 16 == 0 && row_stride % 16 == 0 && sample_offset % 16 == 0 &&
+       (reinterpret_cast<uintptr_t>(d_fpact) & 15) == 0) {
+        switch(tscrunch) {
+        case 4: return launch_ts<4>(args, stream);
+        case 8: return launch_ts<8>(args, stream);
+        case 16: return launch_ts<16>(args, stream);
+        case 32: return launch_ts<32>(args, stream);
+        }
+    }
     const int nout = nsamples / tscrunch;
     dim3 grid(cdiv(nout, 128), nchans);
     if(stokes == 4) {
