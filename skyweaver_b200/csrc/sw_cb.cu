@@ -316,9 +316,10 @@ __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b)
 // scheme, 1.5*2^23 preloaded into TMEM and subtracted in float, and against
 // an integer add of that constant: the plain conversion was fastest, since
 // it needs no TMEM re-arm and no constant registers.)
+template <int DIST = 1>
 __device__ __forceinline__ uint64_t pair_f(const uint32_t* w, int t)
 {
-    return pack2(__int2float_rn((int)w[t]), __int2float_rn((int)w[t + 1]));
+    return pack2(__int2float_rn((int)w[t]), __int2float_rn((int)w[t + DIST]));
 }
 
 // Stokes of L consecutive samples from the exact beam voltages
@@ -329,29 +330,31 @@ __device__ __forceinline__ uint64_t pair_f(const uint32_t* w, int t)
 // packed add that consumes it, every sum is also a single rounding.  (A
 // packed multiply feeding a packed add was measured to be contracted into an
 // FMA, which moved 1 in ~1e5 outputs by one LSB.)
+template <int STOKES>
+__device__ __forceinline__ uint64_t stokes2(uint64_t R0, uint64_t R1, uint64_t I0, uint64_t I1)
+{
+    const uint64_t Z = pack2(0.0f, 0.0f);
+    if constexpr(STOKES <= 1) {
+        const uint64_t E0 = add2(fma2(R0, R0, Z), fma2(I0, I0, Z));  // |p0|^2
+        const uint64_t E1 = add2(fma2(R1, R1, Z), fma2(I1, I1, Z));  // |p1|^2
+        return STOKES == 0 ? add2(E0, E1) : sub2(E0, E1);
+    } else if constexpr(STOKES == 2) {
+        // 2*Re(p0 conj p1) = 2*(r0 r1 - i0 (-i1)) = 2*(r0 r1 + i0 i1)
+        return mul2(add2(fma2(R0, R1, Z), fma2(I0, I1, Z)), pack2(2.0f, 2.0f));
+    } else {
+        // 2*Im(p0 conj p1) = 2*(r0 (-i1) + i0 r1) = 2*(i0 r1 - r0 i1)
+        return mul2(sub2(fma2(I0, R1, Z), fma2(R0, I1, Z)), pack2(2.0f, 2.0f));
+    }
+}
+
 template <int STOKES, int L>
 __device__ __forceinline__ void stokes_n(const uint32_t* r0, const uint32_t* r1,
                                          const uint32_t* i0, const uint32_t* i1, float* st)
 {
-    const uint64_t Z = pack2(0.0f, 0.0f);
 #pragma unroll
-    for(int t = 0; t < L; t += 2) {
-        const uint64_t R0 = pair_f(r0, t), R1 = pair_f(r1, t);
-        const uint64_t I0 = pair_f(i0, t), I1 = pair_f(i1, t);
-        uint64_t S;
-        if constexpr(STOKES <= 1) {
-            const uint64_t E0 = add2(fma2(R0, R0, Z), fma2(I0, I0, Z));  // |p0|^2
-            const uint64_t E1 = add2(fma2(R1, R1, Z), fma2(I1, I1, Z));  // |p1|^2
-            S = STOKES == 0 ? add2(E0, E1) : sub2(E0, E1);
-        } else if constexpr(STOKES == 2) {
-            // 2*Re(p0 conj p1) = 2*(r0 r1 - i0 (-i1)) = 2*(r0 r1 + i0 i1)
-            S = mul2(add2(fma2(R0, R1, Z), fma2(I0, I1, Z)), pack2(2.0f, 2.0f));
-        } else {
-            // 2*Im(p0 conj p1) = 2*(r0 (-i1) + i0 r1) = 2*(i0 r1 - r0 i1)
-            S = mul2(sub2(fma2(I0, R1, Z), fma2(R0, I1, Z)), pack2(2.0f, 2.0f));
-        }
-        unpack2(S, st[t], st[t + 1]);
-    }
+    for(int t = 0; t < L; t += 2)
+        unpack2(stokes2<STOKES>(pair_f(r0, t), pair_f(r1, t), pair_f(i0, t), pair_f(i1, t)),
+                st[t], st[t + 1]);
 }
 
 // All four Stokes parameters (FullStokesBeamformerTraits,
@@ -594,6 +597,12 @@ cb_kernel(const __grid_constant__ Params P)
         // group leave too few registers for it
         constexpr int kG      = (STOKES == 4 && TS <= 4) ? 8 : 16;
         constexpr int kGroups = kSlice / kG;         // column groups per warp
+        // At tscrunch 16 a warp's 32 samples are two outputs: pairing sample t
+        // of one with sample t of the other lets one packed add advance both
+        // power chains (2.17 -> 2.11 ms on 16 channels of the benchmark; at
+        // tscrunch 4 and 8, pairs t and t + tscrunch measured 0-6 % slower).
+        // A column group is then 8 samples of each.
+        constexpr bool kPair  = TS == 16 && STOKES != 4 && !DBG && kSlice == 32;
         const int q   = warp & 3;               // TMEM lane quarter of this warp
         const int h   = ((warp - 2) >> 2) % kHalves;  // which part of the tile's samples
         const int grp = (warp - 2) / (kEpiWarps / 2); // accumulator buffer this warp drains
@@ -658,6 +667,18 @@ cb_kernel(const __grid_constant__ Params P)
                 float power[NC];  // carried across groups while tscrunch > 8
 #pragma unroll
                 for(int c = 0; c < NC; ++c) power[c] = 0.0f;
+                uint64_t power2 = pack2(0.0f, 0.0f);  // kPair: both outputs' chains
+                // one output of a single Stokes parameter
+                auto put = [&](float v, int e) {
+                    if(P.ib_subtract) {
+                        const float ib = kPrefetch ? ibp[kPrefetch ? e : 0] : ibq[e * ib_emit];
+                        v = fsub(v, fmul(ib, 16129.0f));
+                    } else if(STOKES == 0) {
+                        v = fsub(v, offs);
+                    }
+                    const uint32_t o = quant(v);
+                    if(valid) outp[e * out_emit] = (int8_t)o;
+                };
                 // One column group at a time: load, wait, reduce.  (Loading
                 // the next group ahead of the arithmetic, or both groups at
                 // once, was measured 1-2.5 % slower.)
@@ -666,7 +687,17 @@ cb_kernel(const __grid_constant__ Params P)
                 for(int g = 0; g < kGroups; ++g) {
                     uint32_t r0[kG], r1[kG], i0[kG], i1[kG];
                     const uint32_t ta = ta0 + g * kG;
-                    if constexpr(kG == 16) {
+                    if constexpr(kPair) {
+                        const uint32_t tp = ta0 + 8 * g;
+                        SW_TMEM_LD8(tp, r0);
+                        SW_TMEM_LD8(tp + 16, (r0 + 8));
+                        SW_TMEM_LD8(tp + 64, r1);
+                        SW_TMEM_LD8(tp + 64 + 16, (r1 + 8));
+                        SW_TMEM_LD8(tp + 128, i0);
+                        SW_TMEM_LD8(tp + 128 + 16, (i0 + 8));
+                        SW_TMEM_LD8(tp + 192, i1);
+                        SW_TMEM_LD8(tp + 192 + 16, (i1 + 8));
+                    } else if constexpr(kG == 16) {
                         SW_TMEM_LD16(ta, r0);
                         SW_TMEM_LD16(ta + 64, r1);
                         SW_TMEM_LD16(ta + 128, i0);
@@ -697,6 +728,19 @@ cb_kernel(const __grid_constant__ Params P)
                                 make_int2((int)r1[t], (int)i1[t]);
                         }
                     }
+                    if constexpr(kPair) {
+#pragma unroll
+                        for(int t = 0; t < 8; ++t)
+                            power2 = add2(power2, stokes2<STOKES>(pair_f<8>(r0, t), pair_f<8>(r1, t),
+                                                                  pair_f<8>(i0, t), pair_f<8>(i1, t)));
+                        if(g == kGroups - 1) {
+                            float v0, v1;
+                            unpack2(power2, v0, v1);
+                            put(v0, 0);
+                            put(v1, 1);
+                        }
+                        continue;
+                    }
                     float st[NC][kG];
                     if constexpr(STOKES == 4) stokes_iquv<kG>(r0, r1, i0, i1, st);
                     else stokes_n<STOKES, kG>(r0, r1, i0, i1, st[0]);
@@ -709,15 +753,7 @@ cb_kernel(const __grid_constant__ Params P)
                         if(emit) {
                             const int e = u / TS;  // emit index within the slice
                             if constexpr(NC == 1) {
-                                float v = power[0];
-                                if(P.ib_subtract) {
-                                    const float ib = kPrefetch ? ibp[kPrefetch ? e : 0] : ibq[e * ib_emit];
-                                    v = fsub(v, fmul(ib, 16129.0f));
-                                } else if(STOKES == 0) {
-                                    v = fsub(v, offs);
-                                }
-                                const uint32_t o = quant(v);
-                                if(valid) outp[e * out_emit] = (int8_t)o;
+                                put(power[0], e);
                             } else {
                                 // char4 {I, Q, U, V}; the IB power is float4
                                 float v[4] = {power[0], power[1], power[2], power[3]};
