@@ -102,7 +102,13 @@ stats_partial_k(const uint8_t* __restrict__ fpact, size_t row_stride,
 // 8, 4, 2 and 1 heaps per CTA took 0.542, 0.498, 0.526, 0.633 and 1.042 ms,
 // against 0.342 + 0.278 ms for the separate transpose and statistics (16
 // heaps leave a second wave of CTAs that fills a third of the SMs).
+//
+// Shorter gulps give the antenna groups to gridDim.z CTAs, and then fewer heaps
+// to each, until there are kFuseCtas of them (8 CTAs of 256 threads fill an
+// SM): 57 of 64 antennas x 64 channels x 67 heaps 154 -> 140 us, 16 antennas x
+// 8 channels x 16 heaps 24 -> 6 us.
 constexpr int kFuseHeaps = 8;
+constexpr int kFuseCtas  = 8 * 148;
 constexpr int kHeapSamples = 256;
 
 __device__ __forceinline__ uint32_t bperm(uint32_t a, uint32_t b, uint32_t sel)
@@ -119,7 +125,7 @@ transpose_stats_k(const uint4* __restrict__ taftp, uint8_t* __restrict__ fpact,
     const int h0 = blockIdx.x * hpc;
     const int h1 = min(nheaps, h0 + hpc);
     const int c = threadIdx.x & 63, lane = threadIdx.x & 31;
-    for(int ag = 0; ag < out_nant; ag += 4) {
+    for(int ag = 4 * blockIdx.z; ag < out_nant; ag += 4 * gridDim.z) {
         const int a = ag + (int)(threadIdx.x >> 6);  // uniform across a warp
         int s1[2] = {0, 0}, s2[2] = {0, 0};
         long long s3[2] = {0, 0}, s4[2] = {0, 0};
@@ -335,13 +341,17 @@ int sw_transpose_fpact_statistics(const void* d_taftp, void* d_fpact, int nheaps
     const size_t sum_bytes = (size_t)nseries * 4 * sizeof(long long);
     cudaStream_t s = as_cuda(stream);
     SW_CUDA_CHECK(cudaMemsetAsync(d_scratch, 0, sum_bytes, s));
-    dim3 grid(cdiv(nheaps, kFuseHeaps), nchans);
+    int hpc = kFuseHeaps, groups = 1;
+    auto ctas = [&] { return (long long)cdiv(nheaps, hpc) * nchans * groups; };
+    const int most = cdiv(output_nantennas, 4) < 64 ? cdiv(output_nantennas, 4) : 64;
+    while(groups < most && ctas() < kFuseCtas) ++groups;
+    while(hpc > 1 && 2 * ctas() <= kFuseCtas) hpc /= 2;
+    dim3 grid(cdiv(nheaps, hpc), nchans, groups);
     transpose_stats_k<<<grid, 256, 0, s>>>(static_cast<const uint4*>(d_taftp),
                                           static_cast<uint8_t*>(d_fpact), input_nantennas,
                                           output_nantennas, nchans, nheaps, row_stride,
                                           sample_offset,
-                                          static_cast<unsigned long long*>(d_scratch),
-                                          kFuseHeaps);
+                                          static_cast<unsigned long long*>(d_scratch), hpc);
     SW_LAUNCH_CHECK();
     stats_finalize_k<<<cdiv(nseries, 256), 256, 0, s>>>(
         static_cast<const long long*>(d_scratch), reinterpret_cast<float4*>(d_stats), nseries,

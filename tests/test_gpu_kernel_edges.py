@@ -135,3 +135,45 @@ def test_coherent_dedispersion_windows(cuda, n, F, P, A, T, ov, lag, dms, pad):
             assert float(err.max()) <= 0.5 + tol, (dm, float(err.max()))
         f = torch.view_as_complex(dbg[d]).to(torch.complex128)
         assert float((f - ref).abs().max()) <= tol
+
+
+@pytest.mark.parametrize("A,T,ts,S,stokes,sigma", [
+    (1, 16, 16, 1, "I", 8), (3, 48, 4, 1, "Q", 8), (65, 1040, 8, 9, "I", 8), (200, 544, 32, 2, "V", 8),
+    (64, 528, 16, 8, "IQUV", 8), (7, 2064, 4, 3, "IQUV", 60), (64, 512, 8, 2, "I", 90),
+    (70, 64, 32, 1, "U", 90), (16, 32, 4, 5, "I", 127)])
+@pytest.mark.parametrize("weights", ["masks", "large", "fractional"])
+def test_incoherent_beam_runs(cuda, oracle, A, T, ts, S, stokes, sigma, weights):
+    """The 16-sample-run form against the oracle and against the general form
+    (rows off the 16-byte grid) at ragged run counts, antenna counts off the
+    four warps and the chain's table, more beamsets than a pass takes, signals
+    on both sides of the exactness bound and weights that are not whole."""
+    from skyweaver_b200 import stages
+    g = np.random.default_rng(A + T + ts)
+    F = 3
+    ftpa = np.clip(np.rint(g.normal(0, sigma, size=(F, T, 2, A, 2))), -128, 127).astype(np.int8)
+    ftpa[1] = np.clip(ftpa[1].astype(int) * 4, -128, 127)
+    bw = {"masks": g.integers(0, 2, size=(S, A)), "large": g.integers(-900, 901, size=(S, A)),
+          "fractional": g.uniform(0, 1, size=(S, A))}[weights].astype(np.float32)
+    scale = g.uniform(50, 5e4, size=S * F).astype(np.float32)
+    offset = g.uniform(0, 1e5, size=S * F).astype(np.float32)
+    args = [_dev(cuda, x) for x in (scale, offset, bw)]
+    raw_ref, out_ref = oracle.incoherent_beam(ftpa, ts, scale, offset, bw, S, stokes)
+    for stride, off in ((T, 0), (T + 16, 16), (T + 12, 4)):
+        fp = stages.ftpa_to_fpact(_dev(cuda, ftpa), row_stride=stride, offset=off)
+        raw, out = stages.incoherent_beamform(fp, T, ts, *args, offset_samples=off, stokes=stokes)
+        assert np.array_equal(_np(raw), raw_ref), (stride, off)
+        assert np.array_equal(_np(out), out_ref), (stride, off)
+
+
+@pytest.mark.parametrize("H,A_in,A,F", [(1, 1, 4, 1), (1, 13, 16, 3), (9, 62, 64, 2), (67, 57, 64, 5),
+                                        (16, 255, 256, 1), (8, 5, 5, 160)])
+def test_transpose_statistics_splits(cuda, H, A_in, A, F):
+    """The fused pass at every way its launch splits heaps and antenna groups
+    equals the separate stages."""
+    from skyweaver_b200 import stages
+    g = np.random.default_rng(H * A + F)
+    taftp = _dev(cuda, g.integers(-128, 128, size=(H, A_in, F, 256, 2, 2), dtype=np.int8))
+    fp, st = stages.transpose_fpact_statistics(taftp, A)
+    ref = stages.transpose_fpact(taftp, A)
+    assert bool((fp == ref).all())
+    assert np.array_equal(_np(st), _np(stages.statistics(ref, H * 256)), equal_nan=True)
