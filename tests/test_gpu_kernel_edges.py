@@ -177,3 +177,33 @@ def test_transpose_statistics_splits(cuda, H, A_in, A, F):
     ref = stages.transpose_fpact(taftp, A)
     assert bool((fp == ref).all())
     assert np.array_equal(_np(st), _np(stages.statistics(ref, H * 256)), equal_nan=True)
+
+
+@pytest.mark.parametrize("scale,rate,age", [(1e-6, 0.0, 0.0), (3e-5, 1e-9, 3600.0), (20.0, 0.0, 0.0)])
+def test_weights_single_precision_path(cuda, scale, rate, age):
+    """Weights on the single-precision path, near half-integers (phases whose
+    cosine times 127 a is one) and past its range of turns equal the FP64
+    formula (WeightsManager.cu:16-87, clamped to int8), for antenna weights
+    other than 0 and 1 too.  FP64 values within 1e-9 of a half-integer, where
+    the host's and the device's last bits decide, are left out."""
+    from skyweaver_b200 import stages
+    g = np.random.default_rng(11)
+    B, A = 40, 64
+    freqs = np.array([1284e6, 1e9, 544e6 + 0.25])
+    d = np.zeros((B, A, 3), np.float32)
+    d[..., 0] = g.choice([0.0, 1.0, 0.5, -1.0, 1.7, 30.0, 6000.0], size=(B, A))
+    d[..., 1] = g.uniform(-scale, scale, size=(B, A))
+    d[..., 2] = g.uniform(-rate, rate, size=(B, A))
+    # 127 cos(2 pi phase) on half-integers at the second frequency
+    half = np.arccos((g.integers(-127, 127, size=(10, A)) + 0.5) / 127) / (2 * np.pi)
+    d[:10, :, 0], d[:10, :, 1] = 1.0, half / freqs[1]
+    fba, gemm = stages.generate_weights(_dev(cuda, d), _dev(cuda, freqs), 1.7e9 + age, 1.7e9)
+    D = d.astype(np.float64)
+    phase = (age * D[..., 2] + D[..., 1])[None] * freqs[:, None, None]
+    w = np.stack([np.cos(6.283185307179586 * phase) * 127.0 * D[..., 0],
+                  -np.sin(6.283185307179586 * phase) * 127.0 * D[..., 0]], -1)
+    clear = np.abs(np.abs(w - np.rint(w)) - 0.5) > 1e-9
+    assert clear.mean() > 0.999
+    ref = np.clip(np.rint(w), -128, 127).astype(np.int8)
+    assert np.array_equal(_np(fba)[clear], ref[clear])
+    assert np.array_equal(_np(stages.pack_weights(fba)), _np(gemm))
