@@ -553,7 +553,7 @@ cdd_kernel(const __grid_constant__ Args A)
 // twiddles in shared memory, spectrum in registers: cdd_kernel) was bound by
 // shared-memory wavefronts (63 %), issue (61 %) and its CTA-wide barriers:
 // 64 antennas x 64 channels x 65536 samples at DMs 50, 150 and 500 took 9.21 ms
-// that way with 8192 points and take 5.50 ms here; 32 channels x 32768 samples
+// that way with 8192 points and take 5.48 ms here; 32 channels x 32768 samples
 // with 4096 points 2.10 -> 1.33 ms; 48 antennas x 32 channels x 16384 samples,
 // one DM, with 2048 points 0.285 -> 0.207 ms.  With 16 warps of 126 registers per
 // SM no unit is saturated: FMA pipe and shared-memory wavefronts 54 %, issue

@@ -321,12 +321,12 @@ __device__ __forceinline__ void tm_st16(uint32_t addr, const uint32_t* r)
 }
 __device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// x[q] *= w_q (conjugated for the inverse), q = 1 .. 15, w from tensor memory
+// x[q] *= w_q (conjugated for the inverse), q = 1 .. 15, w from tensor memory;
+// the caller has started the load of the first 16 registers into w[0], as long
+// before as its registers allow
 template <bool INV>
-__device__ __forceinline__ void ptwiddle(Pk* x, uint32_t tw)
+__device__ __forceinline__ void ptwiddle(Pk* x, uint32_t tw, uint32_t (*w)[16])
 {
-    uint32_t w[2][16];
-    tm_ld16(tw, w[0]);
 #pragma unroll
     for(int c = 0; c < 4; ++c) {
         uint32_t* v = w[c & 1];
@@ -447,16 +447,19 @@ template <int LOGN, typename F>
 __device__ __forceinline__ void pk_forward(const PkGroup& g, Pk* x, F after_p0)
 {
     using G = PkGeo<LOGN>;
+    uint32_t w[2][16];
+    tm_ld16(g.tm_tw0, w[0]);
     pdft16<false>(x);
-    ptwiddle<false>(x, g.tm_tw0);
+    ptwiddle<false>(x, g.tm_tw0, w);
 #pragma unroll
     for(int q = 0; q < 16; ++q) pk_store(g.p0 + q * G::STEP0, x[q]);
     pk_sync<LOGN>(g);
     after_p0();
+    tm_ld16(g.tm_tw1, w[0]);
 #pragma unroll
     for(int q = 0; q < 16; ++q) x[q] = pk_load(g.p1 + G::off1(q));
     pdft16<false>(x);
-    ptwiddle<false>(x, g.tm_tw1);
+    ptwiddle<false>(x, g.tm_tw1, w);
 #pragma unroll
     for(int q = 0; q < 16; ++q) pk_store(g.p1 + G::off1(q), x[q]);
     __syncwarp();
@@ -502,19 +505,21 @@ __device__ __forceinline__ void pk_inverse(const PkGroup& g, const float4* chirp
                                                          pk2u(v[4 * i + 2], v[4 * i + 3])});
     }
     pass2_inv<G::R2>(x);
+    tm_ld16(g.tm_tw1, w[0]);
 #pragma unroll
     for(int q = 0; q < 16; ++q) pk_store(g.p2 + 16 * q, x[q]);
     __syncwarp();
 #pragma unroll
     for(int q = 0; q < 16; ++q) x[q] = pk_load(g.p1 + G::off1(q));
-    ptwiddle<true>(x, g.tm_tw1);
+    ptwiddle<true>(x, g.tm_tw1, w);
     pdft16<true>(x);
+    tm_ld16(g.tm_tw0, w[0]);
 #pragma unroll
     for(int q = 0; q < 16; ++q) pk_store(g.p1 + G::off1(q), x[q]);
     pk_sync<LOGN>(g);
 #pragma unroll
     for(int q = 0; q < 16; ++q) x[q] = pk_load(g.p0 + q * G::STEP0);
-    ptwiddle<true>(x, g.tm_tw0);
+    ptwiddle<true>(x, g.tm_tw0, w);
     pdft16<true>(x);
 }
 
