@@ -490,7 +490,7 @@ class BeamformerPipeline:
         call("sw_pipeline_outputs", self.h, dm_idx, ctypes.byref(pcb), None, None, None)
         T = self.gulp // self.tscrunch
         shape = (T, self.nchans, self.nbeams) + ((4,) if self.stokes == "IQUV" else ())
-        return _device_view(pcb.value, int(np.prod(shape))).view(torch.int8).reshape(shape)
+        return torch.as_tensor(_Memory(pcb.value, shape, "|i1"), device="cuda")
 
     def voltages(self, dm_idx: int, channels=None):
         """A copy of the last gulp's voltages that fed the beamformers for one
@@ -536,9 +536,15 @@ class BeamformerPipeline:
         return res
 
 
+class _Memory:
+    """Device memory at `ptr` that something else owns, for torch.as_tensor."""
+    __slots__ = ("__cuda_array_interface__",)
+
+    def __init__(self, ptr, shape, typestr):
+        self.__cuda_array_interface__ = {"shape": shape, "typestr": typestr,
+                                         "data": (ptr, False), "version": 3}
+
+
 def _device_view(ptr, nbytes):
     # Build a uint8 CUDA tensor aliasing `ptr` (owned by the pipeline).
-    class _Arr:
-        __cuda_array_interface__ = {"shape": (nbytes,), "typestr": "|u1",
-                                    "data": (ptr, False), "version": 3}
-    return torch.as_tensor(_Arr(), device="cuda")
+    return torch.as_tensor(_Memory(ptr, (nbytes,), "|u1"), device="cuda")
