@@ -207,3 +207,23 @@ def test_weights_single_precision_path(cuda, scale, rate, age):
     ref = np.clip(np.rint(w), -128, 127).astype(np.int8)
     assert np.array_equal(_np(fba)[clear], ref[clear])
     assert np.array_equal(_np(stages.pack_weights(fba)), _np(gemm))
+
+
+@pytest.mark.parametrize("B", [16, 24, 20, 4, 516, 1040])
+@pytest.mark.parametrize("scale", [1.0, 8.0, 3.0, 6.0, 11.313708, 0.25, 1e-35, 1e33, -4.0, 2.9999998])
+def test_incoherent_dedispersion_quantiser(cuda, oracle, B, scale):
+    """Every load width of the dedisperser, partial last lanes, and the
+    divisionless truncation against the oracle's division: scales with many
+    whole quotients, quotients next to whole numbers, saturated ones, negative
+    scales and scales whose reciprocal is subnormal or overflows."""
+    from skyweaver_b200 import stages
+    g = np.random.default_rng(B)
+    F, D, ts, nout, maxd = 11, 3, 2, 37, 9
+    delays = g.integers(0, maxd + 1, size=(D, F)).astype(np.int32)
+    delays[0, 0] = maxd
+    T = maxd + nout * ts
+    tfb = np.rint(g.normal(0, 12, size=(T, F, B))).clip(-128, 127).astype(np.int8)
+    tfb[: T // 3] = 127
+    ref = oracle.idd(tfb, delays, maxd, ts, np.float32(scale))
+    got = stages.incoherent_dedisperse(_dev(cuda, tfb), _dev(cuda, delays), maxd, ts, scale)
+    assert np.array_equal(_np(got), ref)
