@@ -20,10 +20,11 @@
 // Roles (one CTA per SM, persistent over a ragged work queue):
 //   warp 0      TMA producer (weights double buffered, voltages 4 stages)
 //   warp 1      TMEM allocator + single-thread MMA issuer
-//   warps 2..17 epilogue, two groups of 8 taking alternate tiles (group g
-//               drains accumulator buffer g, and frees the tile's voltage
-//               stage once its accumulators are complete); in a group two
-//               warps per TMEM lane quarter, 32 samples of the tile apiece
+//   warps 2..   epilogue, two or three groups of 8 taking the tiles in turn
+//               (a group frees its tile's voltage stage once the accumulators
+//               are complete, and the accumulators once they are in
+//               registers); in a group two warps per TMEM lane quarter, 32
+//               samples of the tile apiece
 // TMEM: 512 columns = 2 accumulator buffers x (D_re 128 | D_im 128).
 // Every wait is bounded by a kernel-wide deadline; on expiry the CTA records
 // DEV_ERR_CB_TIMEOUT in the device error word, stops issuing work, waits
@@ -50,13 +51,19 @@ constexpr int kMaxTilesPerItem = 64;  // default work item: at most 4096 samples
 constexpr int kItemCost = 2;  // tiles that an item's start costs (weights, empty pipeline)
 constexpr int kMaxDm       = 16;
 constexpr int kMaxProblems = 96;
-// Epilogue warps: two groups of 8, one per accumulator buffer, so that each
-// warp reduces 32 samples of every other tile (per-tile overheads are paid
-// once per 32 samples instead of once per 16: measured 2.6 % faster than
-// 16 warps sharing every tile).
-constexpr int kEpiWarps    = 16;
-static_assert(kEpiWarps == 8 || kEpiWarps == 16, "one or two epilogue warps per TMEM lane quarter");
-constexpr int kThreads     = 32 * (2 + kEpiWarps);
+// Epilogue warps: groups of 8 that take the CTA's tiles in turn, so that each
+// warp reduces 32 samples of its group's tiles (per-tile overheads are paid
+// once per 32 samples instead of once per 16: two groups measured 2.6 % faster
+// than 16 warps sharing every tile).  Two groups drain one accumulator buffer
+// each.  At tscrunch 1 .. 4 the many outputs leave the issue slots waiting, and
+// a third group (26 warps of at most 72 registers, 8 TMEM columns per load)
+// fills them: 4.51 -> 4.18 ms at tscrunch 4 on 16 channels of the benchmark; at
+// 8 and 16 two groups stay 4-8 % ahead.  Full Stokes needs the registers.
+template <int TS, int STOKES, bool DBG>
+constexpr int epi_groups() { return TS <= 4 && STOKES != 4 && !DBG ? 3 : 2; }
+template <int TS, int STOKES, bool DBG>
+constexpr int cta_threads() { return 32 * (2 + 8 * epi_groups<TS, STOKES, DBG>()); }
+constexpr int kAccBars     = 6;  // "accumulators ready" barriers: up to 2 per group
 constexpr int kTmemCols    = 512;
 
 struct Problem {
@@ -436,7 +443,7 @@ __device__ __forceinline__ Item decode(const Params& P, int item)
 // production instances carry no debug path (it costs ~20 registers and a
 // branch per load group).
 template <int TS, int STOKES, bool DBG>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(cta_threads<TS, STOKES, DBG>(), 1)
 cb_kernel(const __grid_constant__ Params P)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -454,7 +461,7 @@ cb_kernel(const __grid_constant__ Params P)
     uint64_t* w_full    = v_empty + nvs;
     uint64_t* w_empty   = w_full + nws;
     uint64_t* acc_full  = w_empty + nws;
-    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* acc_empty = acc_full + kAccBars;
     uint64_t* drain     = acc_empty + 2;  // MMA completion on abort
     uint32_t* s_tmem    = reinterpret_cast<uint32_t*>(drain + 1);
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
@@ -463,6 +470,11 @@ cb_kernel(const __grid_constant__ Params P)
     const uint32_t v_full_s = smem_u32(v_full), v_empty_s = smem_u32(v_empty);
     const uint32_t w_full_s = smem_u32(w_full), w_empty_s = smem_u32(w_empty);
     const uint32_t acc_full_s = smem_u32(acc_full), acc_empty_s = smem_u32(acc_empty);
+    // Tile number s of the CTA uses accumulator buffer s mod 2, is reduced by
+    // group s mod kEpi and completes barrier acc_full[s mod kFull], which is
+    // thus waited for by one group, phase after phase.
+    constexpr int kEpi = epi_groups<TS, STOKES, DBG>(), kFull = kEpi == 2 ? 2 : 2 * kEpi;
+    static_assert(kFull <= kAccBars, "barrier carve-up");
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const unsigned long long deadline = globaltimer() + P.timeout_ns;
@@ -470,7 +482,8 @@ cb_kernel(const __grid_constant__ Params P)
     if(threadIdx.x == 0) {
         for(int i = 0; i < nvs; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
         for(int i = 0; i < nws; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], 1); }
-        for(int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kEpiWarps / 2); }
+        for(int i = 0; i < kFull; ++i) mbar_init(&acc_full[i], 1);
+        for(int i = 0; i < 2; ++i) mbar_init(&acc_empty[i], 8);
         mbar_init(drain, 1);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -541,7 +554,7 @@ cb_kernel(const __grid_constant__ Params P)
             // epilogue warps, so its per-tile instruction count bounds how
             // fast the tensor pipe is fed: descriptors are precomputed words
             // and each tile is one straight run of MMAs.
-            int vs = 0, ws = 0, ab = 0;
+            int vs = 0, ws = 0, ab = 0, fb = 0;
             uint32_t vph = 0, wph = 0, aph = 0;
             const int ksteps = P.kbytes / 32;
             const uint32_t a_hi = desc_hi(P.w_sbo16, P.w_layout);
@@ -570,7 +583,8 @@ cb_kernel(const __grid_constant__ Params P)
                     // one commit per tile: the epilogue frees the voltage stage when
                     // it sees the accumulators (a second commit per tile, for the
                     // stage, measured 2.5 % slower)
-                    mma_commit(acc_full_s + 8 * ab);
+                    mma_commit(acc_full_s + 8 * fb);
+                    if(++fb == kFull) fb = 0;
                     if(++vs == nvs) { vs = 0; vph ^= 1; }
                     if(++ab == 2) { ab = 0; aph ^= 1; }
                 }
@@ -590,12 +604,12 @@ cb_kernel(const __grid_constant__ Params P)
         }
     } else {
         // ------------------------------------------------------ epilogue
-        constexpr int kHalves = kEpiWarps / 8;       // warps per TMEM lane quarter and group
+        constexpr int kHalves = 2;                   // warps per TMEM lane quarter and group
         constexpr int kSlice  = kTileT / kHalves;    // samples per warp per tile
         // TMEM columns per load group: 16 (measured 1.5 % faster than 8),
-        // except for full Stokes at tscrunch <= 4, whose many outputs per
-        // group leave too few registers for it
-        constexpr int kG      = (STOKES == 4 && TS <= 4) ? 8 : 16;
+        // except where the registers do not suffice for it (full Stokes at
+        // tscrunch <= 4, three groups)
+        constexpr int kG      = TS <= 4 && !DBG ? 8 : STOKES == 4 && TS <= 4 ? 8 : 16;
         constexpr int kGroups = kSlice / kG;         // column groups per warp
         // At tscrunch 16 a warp's 32 samples are two outputs: pairing sample t
         // of one with sample t of the other lets one packed add advance both
@@ -605,17 +619,17 @@ cb_kernel(const __grid_constant__ Params P)
         constexpr bool kPair  = TS == 16 && STOKES != 4 && !DBG && kSlice == 32;
         const int q   = warp & 3;               // TMEM lane quarter of this warp
         const int h   = ((warp - 2) >> 2) % kHalves;  // which part of the tile's samples
-        const int grp = (warp - 2) / (kEpiWarps / 2); // accumulator buffer this warp drains
+        const int grp = (warp - 2) / 8;
         const int F = P.nchans;
         const int nout = P.nsamples / TS;
         const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
-        // release this group's accumulator buffer to the MMA warp (phase 0)
+        // the first two groups release the accumulator buffers to the MMA warp
+        // (phase 0)
         fence_before();
         __syncwarp();
-        if(lane == 0) mbar_arrive(&acc_empty[grp]);
-        int ab = 0;        // accumulator buffer of the CTA's next tile
+        if(lane == 0 && grp < 2) mbar_arrive(&acc_empty[grp]);
         int seq = 0;       // CTA tile sequence number of the item's first tile
-        uint32_t aph = 0;  // phase parity of this group's buffer
+        int mine = grp;    // that of this group's next tile
         for(int item = blockIdx.x; item < P.nitems && !*s_abort; item += gridDim.x) {
             const Item it = decode(P, item);
             const Problem& pr = P.prob[it.p];
@@ -626,14 +640,13 @@ cb_kernel(const __grid_constant__ Params P)
             const float offs  = P.offset[bs * F + it.f];
             const int tile0 = it.tc * P.tpi;
             const int tile1 = min(ntiles_gulp, tile0 + P.tpi);
-            // tiles alternate between the buffers: this group takes every
-            // other tile, starting with the first one that lands in its buffer
-            const int first = tile0 + ((ab ^ grp) & 1);
+            // the groups take the tiles in turn, across item boundaries
+            const int first = tile0 + mine - seq;
             bool ok = true;
             constexpr int NC = STOKES == 4 ? 4 : 1;  // output components
             constexpr int kEmits = kSlice / TS;      // outputs per warp per tile
             // Output and IB-power elements of this warp's first output in
-            // its first tile; both advance by 2 kTileT / TS output samples.
+            // its first tile; both advance by kEpi kTileT / TS output samples.
             const int to0 = (first * kTileT + h * kSlice) / TS;
             int8_t* outp = pr.out + (((size_t)to0 * F + it.f) * P.nbeams + b) * NC;
             const float* ibq =
@@ -644,7 +657,10 @@ cb_kernel(const __grid_constant__ Params P)
             // accumulator wait so that their latency hides behind it
             constexpr bool kPrefetch = kEmits * NC <= 4;
             float ibp[kPrefetch ? kEmits * NC : 1];
-            for(int tile = first; tile < tile1; tile += 2) {
+            for(int tile = first; tile < tile1; tile += kEpi, mine += kEpi) {
+                const int buf = kEpi == 2 ? grp : mine & 1;
+                const int full = kEpi == 2 ? grp : mine % kFull;
+                const uint32_t fph = (kEpi == 2 ? mine / 2 : mine / kFull) & 1;
                 if constexpr(kPrefetch) {
                     if(P.ib_subtract) {
 #pragma unroll
@@ -659,10 +675,9 @@ cb_kernel(const __grid_constant__ Params P)
                         }
                     }
                 }
-                if(!mbar_wait(acc_full_s + 8 * grp, aph, s_abort, deadline, P.err)) { ok = false; break; }
+                if(!mbar_wait(acc_full_s + 8 * full, fph, s_abort, deadline, P.err)) { ok = false; break; }
                 // the tile's MMAs are complete, so its voltage stage is free
-                if(warp == 2 + (kEpiWarps / 2) * grp && lane == 0)
-                    mbar_arrive(&v_empty[(seq + tile - tile0) % nvs]);
+                if(warp == 2 + 8 * grp && lane == 0) mbar_arrive(&v_empty[mine % nvs]);
                 fence_after();
                 float power[NC];  // carried across groups while tscrunch > 8
 #pragma unroll
@@ -682,7 +697,7 @@ cb_kernel(const __grid_constant__ Params P)
                 // One column group at a time: load, wait, reduce.  (Loading
                 // the next group ahead of the arithmetic, or both groups at
                 // once, was measured 1-2.5 % slower.)
-                const uint32_t ta0 = lane_base + grp * 256 + h * kSlice;
+                const uint32_t ta0 = lane_base + buf * 256 + h * kSlice;
 #pragma unroll
                 for(int g = 0; g < kGroups; ++g) {
                     uint32_t r0[kG], r1[kG], i0[kG], i1[kG];
@@ -715,7 +730,7 @@ cb_kernel(const __grid_constant__ Params P)
                         // instead: 2.40 against 2.11 ms at tscrunch 16)
                         fence_before();
                         __syncwarp();
-                        if(lane == 0) mbar_arrive(&acc_empty[grp]);
+                        if(lane == 0) mbar_arrive(&acc_empty[buf]);
                     }
                     const int tbase = tile * kTileT + h * kSlice + g * kG;
                     if(DBG && valid) {
@@ -777,12 +792,10 @@ cb_kernel(const __grid_constant__ Params P)
                         }
                     }
                 }
-                aph ^= 1;
-                outp += (2 * kTileT / TS) * out_emit;
-                if(P.ib_subtract) ibq += (2 * kTileT / TS) * ib_emit;
+                outp += (kEpi * kTileT / TS) * out_emit;
+                if(P.ib_subtract) ibq += (kEpi * kTileT / TS) * ib_emit;
             }
             if(!ok) break;
-            ab ^= (tile1 - tile0) & 1;
             seq += tile1 - tile0;
         }
     }
@@ -867,7 +880,7 @@ int dispatch_ts(int ts, int stokes, int grid, size_t smem, cudaStream_t stream);
 size_t smem_bytes(int kbytes, int vstages, int wstages)
 {
     return 1024 + (size_t)wstages * 2 * kM * kbytes + (size_t)vstages * 2 * kbytes * kTileT +
-           (2 * vstages + 2 * wstages + 5) * 8 + 16;
+           (2 * vstages + 2 * wstages + kAccBars + 3) * 8 + 16;
 }
 
 int num_sms()
@@ -1018,7 +1031,7 @@ int launch_instance(int grid, size_t smem, cudaStream_t stream)
 {
     SW_CUDA_CHECK(cudaFuncSetAttribute(cb_kernel<TS, STOKES, DBG>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cb_kernel<TS, STOKES, DBG><<<grid, kThreads, smem, stream>>>(launch_params());
+    cb_kernel<TS, STOKES, DBG><<<grid, cta_threads<TS, STOKES, DBG>(), smem, stream>>>(launch_params());
     SW_LAUNCH_CHECK();
     return SW_OK;
 }
