@@ -22,8 +22,10 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel)
 }
 
 // ---------------------------------------------------------------------------
-// TAFTP -> FTPA.  One CTA per (heap, channel).  The heap's A_in x 256 x P
-// char2 block (1 KiB per antenna) is staged in shared memory as 32-bit words
+// TAFTP -> FTPA.  One CTA per (half heap, channel): 29 KiB of shared memory for
+// 57 antennas, so that several CTAs per SM overlap their loads and stores
+// (57 of 64 antennas x 16 channels x 32 heaps: 12.6 us; whole heaps 23 us).  The half heap's A_in x 128 x P char2 block (512 bytes
+// per antenna) is staged in shared memory as 32-bit words
 // w[a][s] = (p0.re, p0.im, p1.re, p1.im); the word index within a row is
 // XOR-swizzled by the antenna group so that the column reads below are
 // bank-conflict free.  Each thread then emits 16-byte output chunks
@@ -31,7 +33,7 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int swz_word(int a, int s)
 {
-    return a * kHeap + (s ^ (((a >> 3) & 7) << 2));
+    return a * (kHeap / 2) + (s ^ (((a >> 3) & 7) << 2));
 }
 
 __global__ void __launch_bounds__(256)
@@ -41,10 +43,11 @@ transpose_ftpa_k(const uint4* __restrict__ taftp, uint4* __restrict__ ftpa,
     extern __shared__ uint32_t sm_words[];
     const int h = blockIdx.x;
     const int f = blockIdx.y;
-    // stage: A_in x 64 chunks of 16 bytes (4 samples x 2 pols x char2)
-    for(int idx = threadIdx.x; idx < in_nant * 64; idx += blockDim.x) {
-        const int a = idx >> 6, c = idx & 63;
-        const size_t src = (((size_t)h * in_nant + a) * nchans + f) * 64 + c;
+    const int z = blockIdx.z;  // half of the heap
+    // stage: A_in x 32 chunks of 16 bytes (4 samples x 2 pols x char2)
+    for(int idx = threadIdx.x; idx < in_nant * 32; idx += blockDim.x) {
+        const int a = idx >> 5, c = idx & 31;
+        const size_t src = (((size_t)h * in_nant + a) * nchans + f) * 64 + 32 * z + c;
         uint4 v = taftp[src];
         uint4* dst = reinterpret_cast<uint4*>(&sm_words[swz_word(a, c * 4)]);
         *dst = v;
@@ -52,7 +55,7 @@ transpose_ftpa_k(const uint4* __restrict__ taftp, uint4* __restrict__ ftpa,
     __syncthreads();
     const int groups = out_nant >> 3;  // 8 antennas -> 16 bytes per row
     const size_t nsamp = (size_t)nheaps * kHeap;
-    for(int idx = threadIdx.x; idx < groups * kHeap; idx += blockDim.x) {
+    for(int idx = threadIdx.x; idx < groups * (kHeap / 2); idx += blockDim.x) {
         const int g = idx % groups;
         const int s = idx / groups;
         uint32_t w[8];
@@ -66,7 +69,7 @@ transpose_ftpa_k(const uint4* __restrict__ taftp, uint4* __restrict__ ftpa,
         o0.y = prmt(w[2], w[3], 0x5410); o1.y = prmt(w[2], w[3], 0x7632);
         o0.z = prmt(w[4], w[5], 0x5410); o1.z = prmt(w[4], w[5], 0x7632);
         o0.w = prmt(w[6], w[7], 0x5410); o1.w = prmt(w[6], w[7], 0x7632);
-        const size_t t   = (size_t)h * kHeap + s;
+        const size_t t   = (size_t)h * kHeap + z * (kHeap / 2) + s;
         const size_t row = ((size_t)f * nsamp + t) * kPol;  // (f, t, p=0)
         // row of out_nant char2 = out_nant/8 uint4
         ftpa[row * groups + g]           = o0;
@@ -119,7 +122,7 @@ transpose_fpact_k(const uint4* __restrict__ taftp, uint8_t* __restrict__ fpact,
 // (sample t, column w) lies at column w ^ (t / 4 mod 32), which keeps both
 // the accesses along w and those along t (4 samples apart) free of bank
 // conflicts.  Bound by HBM: 57 -> 64 antennas x 16 channels x 8192 samples
-// took 287 us with a byte access per value and takes 20 us so.
+// took 287 us with a byte access per value and takes 26 us so.
 // Bases, strides or offsets off the 4-byte grid take the byte accesses of
 // `row_words` = 0, as does a last group of fewer than 4 samples.
 constexpr int kConvT = 128, kConvW = 64;
@@ -229,11 +232,11 @@ int sw_transpose_ftpa(const void* d_taftp, void* d_ftpa, int nheaps,
     SW_REQUIRE(output_nantennas % 8 == 0 && output_nantennas <= 256,
                "sw_transpose_ftpa: output antennas must be a multiple of 8 and <= 256");
     SW_REQUIRE(nheaps <= 65535 && nchans <= 65535, "sw_transpose_ftpa: grid too large");
-    const size_t smem = (size_t)input_nantennas * kHeap * 4;
+    const size_t smem = (size_t)input_nantennas * (kHeap / 2) * 4;
     SW_CUDA_CHECK(cudaFuncSetAttribute(transpose_ftpa_k,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem));
-    dim3 grid(nheaps, nchans);
+    dim3 grid(nheaps, nchans, 2);
     transpose_ftpa_k<<<grid, 256, smem, as_cuda(stream)>>>(
         static_cast<const uint4*>(d_taftp), static_cast<uint4*>(d_ftpa),
         input_nantennas, output_nantennas, nchans, nheaps);
