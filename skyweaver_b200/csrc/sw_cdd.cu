@@ -679,7 +679,12 @@ cdd_pk_kernel(const __grid_constant__ Args A)
 // the overlap-save trim, /N, rint and int8 wrap.  DMs of exactly 0 are copied
 // from the rows by the combine step.
 // 64 antennas x 8 channels x 65536 samples at 65536 points and DMs 0, 50, 150
-// and 500: 7.46 ms with 16 points a thread in scalar arithmetic, 4.12 ms so.
+// and 500: 7.46 ms with 16 points a thread in scalar arithmetic, 4.12 ms with
+// these sub-transforms, 2.72 ms with the rows loaded without a branch between
+// the loads (before, each waited for the last), 2.64 ms with pairs stored
+// whole.  A cluster of S CTAs that combines from each other's shared memory
+// instead of through the workspace took 3.58 ms: 15 clusters of 8 run at once,
+// and its barriers tie both windows of a CTA together.
 constexpr int kSplitLog = 13;
 constexpr int kSplitM   = 1 << kSplitLog;
 
@@ -729,7 +734,8 @@ cdd_split_kernel(const __grid_constant__ SplitArgs A)
     const int t = g.t;
     const int L = N - A.overlap;
     const int avail = A.overlap + A.nsamples;
-    const bool even = ((L | (int)(A.row_stride & 1)) & 1) == 0 &&
+    // pairs of samples are aligned, and inside the rows or past them together
+    const bool even = ((L | avail | (int)(A.row_stride & 1)) & 1) == 0 &&
                       (reinterpret_cast<uintptr_t>(A.in) & 1) == 0;
 
     const int nunits = A.nitems * S;
@@ -752,24 +758,40 @@ cdd_split_kernel(const __grid_constant__ SplitArgs A)
             const Pk wp = {pk2(w.x, w.x), pk2(w.y, w.y)};
             const int left = avail - (start + n1 * M + 2 * t);  // samples from this thread's first
             if(avail - (start + n1 * M) <= 0) break;            // zero padding from here on
+            // all loads of 8 pairs in flight at once: no branch between them (pairs
+            // past the end read the row's first samples and count as zeros)
 #pragma unroll
-            for(int r = 0; r < 16; ++r) {
-                const int at = n1 * M + 512 * r;
-                uint32_t re = 0, im = 0;
-                if(even && 512 * r + 1 < left) {
-                    re = *reinterpret_cast<const uint16_t*>(row_re + at);
-                    im = *reinterpret_cast<const uint16_t*>(row_im + at);
+            for(int h = 0; h < 16; h += 8) {
+                uint32_t re[8], im[8];
+                if(even) {
+#pragma unroll
+                    for(int i = 0; i < 8; ++i) {
+                        const bool in = 512 * (h + i) < left;
+                        const int at  = in ? n1 * M + 512 * (h + i) : -2 * t;
+                        const uint32_t a = *reinterpret_cast<const uint16_t*>(row_re + at);
+                        const uint32_t b = *reinterpret_cast<const uint16_t*>(row_im + at);
+                        re[i] = in ? a : 0;
+                        im[i] = in ? b : 0;
+                    }
                 } else {
-                    if(512 * r < left) { re = row_re[at]; im = row_im[at]; }
-                    if(512 * r + 1 < left) {
-                        re |= (uint32_t)row_re[at + 1] << 8;
-                        im |= (uint32_t)row_im[at + 1] << 8;
+                    for(int i = 0; i < 8; ++i) {
+                        const int at = n1 * M + 512 * (h + i);
+                        re[i] = im[i] = 0;
+                        if(512 * (h + i) < left) { re[i] = row_re[at]; im[i] = row_im[at]; }
+                        if(512 * (h + i) + 1 < left) {
+                            re[i] |= (uint32_t)row_re[at + 1] << 8;
+                            im[i] |= (uint32_t)row_im[at + 1] << 8;
+                        }
                     }
                 }
-                const uint64_t xr = pk2((float)(int8_t)re, (float)(int8_t)(re >> 8));
-                const uint64_t xi = pk2((float)(int8_t)im, (float)(int8_t)(im >> 8));
-                x[r].re = psub(pfma(xr, wp.re, x[r].re), pmul(xi, wp.im));
-                x[r].im = pfma(xi, wp.re, pfma(xr, wp.im, x[r].im));
+#pragma unroll
+                for(int i = 0; i < 8; ++i) {
+                    const uint64_t xr = pk2((float)(int8_t)re[i], (float)(int8_t)(re[i] >> 8));
+                    const uint64_t xi = pk2((float)(int8_t)im[i], (float)(int8_t)(im[i] >> 8));
+                    Pk& v = x[h + i];
+                    v.re = psub(pfma(xr, wp.re, v.re), pmul(xi, wp.im));
+                    v.im = pfma(xi, wp.re, pfma(xr, wp.im, v.im));
+                }
             }
         }
         const float4* tws = A.tws + (size_t)k1 * (M / 2) + t;
@@ -813,6 +835,10 @@ cdd_split_combine(const __grid_constant__ SplitArgs A)
     const float inv_n = 1.0f / (float)N;  // exact (power of two)
     // as in cdd_pk_kernel: the low byte of v / N + 1.5 2^23 is the sample
     const uint64_t scale = pk2(inv_n, inv_n), magic = pk2(12582912.0f, 12582912.0f);
+    // both samples of a pair are kept or trimmed together, at even places
+    const bool even = ((L | head | A.nsamples) & 1) == 0 && (A.out_stride & 1) == 0;
+    const bool even_in = even && (A.row_stride & 1) == 0 &&
+                         (reinterpret_cast<uintptr_t>(A.in) & 1) == 0;
     const size_t total = (size_t)A.ndms * A.nitems * (M / 2);
     for(size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
         idx += (size_t)gridDim.x * blockDim.x) {
@@ -829,6 +855,19 @@ cdd_split_combine(const __grid_constant__ SplitArgs A)
         uint8_t* o_im = o_re + A.out_stride;
         if(A.zero_flags[d] && !A.dbg) {
             const uint8_t* i_re = A.in + (size_t)stream * 2 * A.row_stride + start + head;
+            if(even_in && (reinterpret_cast<uintptr_t>(A.out[d]) & 1) == 0) {
+#pragma unroll
+                for(int n1 = 0; n1 < S; ++n1) {
+                    const int v = n2 + n1 * M - head;
+                    if((unsigned)v < kept) {
+                        *reinterpret_cast<uint16_t*>(o_re + v) =
+                            *reinterpret_cast<const uint16_t*>(i_re + v);
+                        *reinterpret_cast<uint16_t*>(o_im + v) =
+                            *reinterpret_cast<const uint16_t*>(i_re + A.row_stride + v);
+                    }
+                }
+                continue;
+            }
             for(int n1 = 0; n1 < S; ++n1)
                 for(int e = 0; e < 2; ++e) {
                     const int v = n2 + e + n1 * M - head;
@@ -847,12 +886,22 @@ cdd_split_combine(const __grid_constant__ SplitArgs A)
             z[k1] = {pk2(re.x, re.y), pk2(im.x, im.y)};
         }
         pdft<S, true>(z);  // z[n1] = sum_k1 W_S^(-n1 k1) z'[k1]
+        const bool words = even && !A.dbg && (reinterpret_cast<uintptr_t>(A.out[d]) & 1) == 0;
 #pragma unroll
         for(int n1 = 0; n1 < S; ++n1) {
             const int v = n2 + n1 * M - head;
             uint32_t re[2], im[2];
             unpk2u(pfma(z[n1].re, scale, magic), re[0], re[1]);
             unpk2u(pfma(z[n1].im, scale, magic), im[0], im[1]);
+            if(words) {
+                if((unsigned)v < kept) {
+                    *reinterpret_cast<uint16_t*>(o_re + v) =
+                        (uint16_t)__byte_perm(re[0], re[1], 0x0040);
+                    *reinterpret_cast<uint16_t*>(o_im + v) =
+                        (uint16_t)__byte_perm(im[0], im[1], 0x0040);
+                }
+                continue;
+            }
             float fr[2], fi[2];
             unpk2(pmul(z[n1].re, scale), fr[0], fr[1]);
             unpk2(pmul(z[n1].im, scale), fi[0], fi[1]);

@@ -24,8 +24,9 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel)
 // ---------------------------------------------------------------------------
 // TAFTP -> FTPA.  One CTA per (half heap, channel): 29 KiB of shared memory for
 // 57 antennas, so that several CTAs per SM overlap their loads and stores
-// (57 of 64 antennas x 16 channels x 32 heaps: 12.6 us; whole heaps 23 us).  The half heap's A_in x 128 x P char2 block (512 bytes
-// per antenna) is staged in shared memory as 32-bit words
+// (57 of 64 antennas x 16 channels x 32 heaps: 12.6 us; whole heaps 23 us).
+// The half heap's A_in x 128 x P char2 block (512 bytes per antenna) is staged
+// in shared memory as 32-bit words
 // w[a][s] = (p0.re, p0.im, p1.re, p1.im); the word index within a row is
 // XOR-swizzled by the antenna group so that the column reads below are
 // bank-conflict free.  Each thread then emits 16-byte output chunks
