@@ -182,23 +182,27 @@ extern "C" int sw_autotune(int nantennas, int nbeams, int nchans, int nsamples, 
                                                 static_cast<int*>(map.p), stream);
         }, s, 3, ms);
     };
-    // work-item size (the tile's extent in time) at the default depths ...
-    for(int tpi : {4, 8, 16, 32, 64, 128}) {
-        if(tpi > T / 64 && tpi != 4) break;
+    // work-item size (the tile's extent in time) at the default depths, and then
+    // the depths, starting from what a launch takes by default; another choice
+    // has to be 2 % faster, which is more than three repetitions scatter
+    // (choices within the scatter picked 128 tiles and 3 stages for the
+    // benchmark, 1-3 % behind the default in long runs)
+    const float kGain = 0.98f;
+    for(int tpi : {64, 4, 8, 16, 32, 128}) {
+        if(tpi > T / 64 && tpi != 4) continue;
         float ms = 0.0f;
         SW_TRY(time_cb(tpi, 4, 2, &ms));
-        if(ms < best.cb_ms) {
+        if(ms < kGain * best.cb_ms) {
             best.cb_ms = ms;
             best.cb_tiles_per_item = tpi;
             best.cb_voltage_stages = 4;
             best.cb_weight_stages = 2;
         }
     }
-    // ... then the pipeline depths at that size
     for(auto vw : {std::pair<int, int>{2, 2}, {3, 2}, {6, 2}, {8, 2}, {4, 3}, {6, 3}}) {
         float ms = 0.0f;
         SW_TRY(time_cb(best.cb_tiles_per_item, vw.first, vw.second, &ms));
-        if(ms < best.cb_ms) {
+        if(ms < kGain * best.cb_ms) {
             best.cb_ms = ms;
             best.cb_voltage_stages = vw.first;
             best.cb_weight_stages = vw.second;

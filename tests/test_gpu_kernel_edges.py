@@ -115,7 +115,8 @@ def test_coherent_dedispersion_windows(cuda, n, F, P, A, T, ov, lag, dms, pad):
     outs = [torch.full((F, P, A, 2, T + pad), 99, dtype=torch.int8, device="cuda") for _ in dms]
     plain = [o.clone() for o in outs]
     _, dbg = cdd.dedisperse(ext, T, outs=outs, debug=True)
-    cdd.dedisperse(ext, T, outs=plain)
+    # long windows: one at a time through the smallest workspace
+    cdd.dedisperse(ext, T, outs=plain, workspace_limit=1)
     z = torch.complex(ext[..., 0, :ov + T].double(), ext[..., 1, :ov + T].double())
     step = n - ov
     for d, dm in enumerate(dms):
