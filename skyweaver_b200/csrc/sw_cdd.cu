@@ -6,19 +6,21 @@
 // DMResponse (:293-336) and the golden-vector generator
 // python/skyweaver_test_utils/dedisperse.py:58-80,143-173.
 //
-// B200 design: one CTA transforms one overlap-save segment of one
-// (channel, pol, antenna) stream entirely in shared memory and registers:
-//   * the forward FFT is an in-place mixed-radix decimation-in-frequency
-//     FFT (first pass radix 2/4/8/16 read straight from the planar int8
-//     rows, then radix-16 passes); its last pass leaves each thread's 16
-//     spectral bins in registers, in digit-reversed order;
-//   * for every coherent DM the thread multiplies those bins by the chirp
-//     (FP64 phases, stored as complex float in the same digit-reversed
-//     order), runs the exact inverse passes (decimation in time, conjugate
-//     twiddles) and the last pass writes the trimmed, scaled, rounded and
-//     int8-wrapped samples straight to the planar output rows.
-// So the forward transform is done once per segment for all DMs, there is
-// no spectrum in HBM, and all global traffic is coalesced byte rows.
+// B200 design: one overlap-save window of one (channel, pol, antenna) stream is
+// transformed entirely on chip, for 1024 to 8192 points by a group of N / 32
+// threads in packed pairs (sw_cdd_pk.cuh, cdd_pk_kernel), for 256 and 512 points
+// by a CTA of N / 16 threads (cdd_kernel); longer windows are split into
+// 8192-point sub-transforms (cdd_split_kernel):
+//   * the forward FFT is in place, decimation in frequency, its first pass read
+//     straight from the staged planar int8 rows, its last pass leaving each
+//     thread's spectral bins in registers in digit-reversed order;
+//   * for every coherent DM the thread multiplies its bins by the chirp (FP64
+//     phases, stored as complex float in the order the threads load it), runs
+//     the exact inverse passes (decimation in time, conjugate twiddles), and
+//     the last pass writes the trimmed, scaled, rounded and int8-wrapped
+//     samples straight to the planar output rows.
+// So the forward transform is done once per window for all DMs, there is no
+// spectrum in HBM (up to 8192 points), and all global traffic is coalesced.
 //
 // Trim.  The reference trims overlap/2 samples at each end of a window.  Its
 // chirp's impulse response is one-sided (nearly all of it at lags 0 .. the
@@ -26,8 +28,7 @@
 // start (the causal part) and `lag` at its end (the short anti-causal part);
 // output sample m is the dedispersed voltage at gulp position m - lag.
 // lag = overlap / 2 is the reference's own per-window trim.
-// Twiddles come from per-pass tables (FP64-computed) staged in shared
-// memory; FFT arithmetic is FP32.
+// Twiddles come from FP64-computed tables; FFT arithmetic is FP32.
 #include <algorithm>
 
 #include "sw_cdd_pk.cuh"
@@ -172,39 +173,11 @@ __device__ __forceinline__ void dft16(c32* x)
     for(int i = 0; i < 16; ++i) x[i] = t[i];
 }
 
-template <bool INV>
-__device__ __forceinline__ void dft8(c32* x)
-{
-    // radix 2 x 4: r = 4*r1 + r2, q = q1 + 2*q2
-#pragma unroll
-    for(int r2 = 0; r2 < 4; ++r2) {
-        c32 a = x[r2], b = x[4 + r2];
-        x[r2] = cadd(a, b);
-        x[4 + r2] = csub(a, b);
-    }
-    // twiddle W8^(r2*q1) on the q1 = 1 half
-    const float c2 = 0.70710678118654752440f;
-    x[5] = cmul(x[5], c32{c2, INV ? c2 : -c2});
-    x[6] = rot90<INV>(x[6]);
-    x[7] = cmul(x[7], c32{-c2, INV ? c2 : -c2});
-    dft4<INV>(x[0], x[1], x[2], x[3]);
-    dft4<INV>(x[4], x[5], x[6], x[7]);
-    c32 t[8];
-#pragma unroll
-    for(int q2 = 0; q2 < 4; ++q2) {
-        t[2 * q2]     = x[q2];
-        t[2 * q2 + 1] = x[4 + q2];
-    }
-#pragma unroll
-    for(int i = 0; i < 8; ++i) x[i] = t[i];
-}
-
 template <int R, bool INV>
 __device__ __forceinline__ void dft(c32* x)
 {
+    static_assert(R == 16 || R == 2, "256 = 16 x 16, 512 = 2 x 16 x 16");
     if constexpr(R == 16) dft16<INV>(x);
-    else if constexpr(R == 8) dft8<INV>(x);
-    else if constexpr(R == 4) dft4<INV>(x[0], x[1], x[2], x[3]);
     else dft2<INV>(x);
 }
 

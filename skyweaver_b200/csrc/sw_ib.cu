@@ -282,10 +282,28 @@ __device__ __noinline__ float ib_chain(const IbArgs& args, int f, int t0, const 
                     v[2][k] = *reinterpret_cast<const uint32_t*>(p1 + 2 * a * rs + tc + 4 * k);
                     v[3][k] = *reinterpret_cast<const uint32_t*>(p1 + (2 * a + 1) * rs + tc + 4 * k);
                 }
+                if(stokes == 0) {
+                    // Stokes I of int8 voltages is a whole number below 2^17, so
+                    // the reference's float steps are exact: the four bytes of a
+                    // sample (PRMT transpose) summed as squares by one dp4a
 #pragma unroll
-                for(int k = 0; k < L; ++k) {
-                    auto byte = [&](int r) { return (float)(int8_t)(v[r][k / 4] >> (8 * (k & 3))); };
-                    x[k][a] = fmul(stokes_f(stokes, byte(0), byte(1), byte(2), byte(3)), w[a]);
+                    for(int k = 0; k < L / 4; ++k) {
+                        const uint32_t t0 = __byte_perm(v[0][k], v[1][k], 0x5140);
+                        const uint32_t t1 = __byte_perm(v[2][k], v[3][k], 0x5140);
+                        const uint32_t t2 = __byte_perm(v[0][k], v[1][k], 0x7362);
+                        const uint32_t t3 = __byte_perm(v[2][k], v[3][k], 0x7362);
+                        const uint32_t s[4] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632),
+                                               __byte_perm(t2, t3, 0x5410), __byte_perm(t2, t3, 0x7632)};
+#pragma unroll
+                        for(int i = 0; i < 4; ++i)
+                            x[4 * k + i][a] = fmul((float)__dp4a((int)s[i], (int)s[i], 0), w[a]);
+                    }
+                } else {
+#pragma unroll
+                    for(int k = 0; k < L; ++k) {
+                        auto byte = [&](int r) { return (float)(int8_t)(v[r][k / 4] >> (8 * (k & 3))); };
+                        x[k][a] = fmul(stokes_f(stokes, byte(0), byte(1), byte(2), byte(3)), w[a]);
+                    }
                 }
             }
             for(int k = 0; k < L; ++k)
