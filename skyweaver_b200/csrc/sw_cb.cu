@@ -475,7 +475,14 @@ cb_kernel(const __grid_constant__ Params P)
     // thus waited for by one group, phase after phase.
     constexpr int kEpi = epi_groups<TS, STOKES, DBG>(), kFull = kEpi == 2 ? 2 : 2 * kEpi;
     static_assert(kFull <= kAccBars, "barrier carve-up");
-    const int warp = threadIdx.x >> 5;
+    // With two epilogue groups the warp index and the TMEM base pass through a
+    // shuffle, so that the compiler holds them and the addresses made from them
+    // once per warp: 2.50 -> 2.35 ms at tscrunch 8, 2.10 -> 2.04 at 16 (16
+    // channels of 65536 samples, 1024 beams, 4 DMs).  With three it costs
+    // (4.3 -> 4.5 ms at tscrunch 4), and both stay plain.
+    constexpr bool kUniform = kEpi == 2;
+    int warp = threadIdx.x >> 5;
+    if constexpr(kUniform) { warp = __shfl_sync(0xffffffffu, warp, 0); }
     const int lane = threadIdx.x & 31;
     const unsigned long long deadline = globaltimer() + P.timeout_ns;
 
@@ -497,7 +504,8 @@ cb_kernel(const __grid_constant__ Params P)
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = *s_tmem;
+    uint32_t tmem = *s_tmem;
+    if constexpr(kUniform) { tmem = __shfl_sync(0xffffffffu, tmem, 0); }
     const int ntiles_gulp = P.nsamples / kTileT;
 
     if(warp == 0) {
