@@ -245,7 +245,11 @@ constexpr int kIbWarps = 4;
 // The reference's float chain (t outer, a inner, float multiply and add) of
 // one output, from a table of its products (see ib_k), or sample by sample
 // when the antennas exceed the table.  First decides in 64 bits whether this
-// beamset's own sum is exact after all (`sum` holds it).
+// beamset's own sum is exact after all (`sum` holds it).  Stokes I of int8
+// samples is a whole number below 2^17, exact in float: the table takes it
+// from a byte transpose and one dp4a a sample in place of four conversions
+// and seven float operations, 240 -> 225 us per DM for 64 antennas, 64
+// channels of 65536 samples, three of them on the chain.
 template <int TS>
 __device__ __noinline__ float ib_chain(const IbArgs& args, int f, int t0, const float* w,
                                        bool int_weights, int stokes, int sum)
