@@ -346,7 +346,8 @@ int sw_coherent_dedisperse_channel(const void* d_fpact_in, size_t row_stride,
  * (cpp/skyweaver/IncoherentDedisperser.cuh:24-26,
  *  cpp/skyweaver/src/IncoherentDedisperser.cu:66-125) on the GPU.
  * d_delays: int [ndms][nchans] sample delays; scale_factor as the
- * reference's prepare() computes it. */
+ * reference's prepare() computes it.  nbeams a multiple of 4, d_tfb and d_tdb
+ * aligned to 4 bytes (fastest with all three multiples of 16). */
 int sw_incoherent_dedisperse(const int8_t* d_tfb, int nsamples, int nchans,
                              int nbeams, const int* d_delays, int ndms,
                              int max_delay, int tscrunch, float scale_factor,

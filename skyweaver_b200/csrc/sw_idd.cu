@@ -259,12 +259,15 @@ extern "C" int sw_incoherent_dedisperse(const int8_t* d_tfb, int nsamples,
                "(nsamples - max_sample_delay) must be a multiple of tscrunch;");
     SW_REQUIRE(nbeams % 4 == 0, "sw_incoherent_dedisperse: nbeams must be a multiple of 4");
     SW_REQUIRE(ndms > 0 && ndms <= 65535, "sw_incoherent_dedisperse: bad DM count");
-    const int nout = (nsamples - max_delay) / tscrunch;
     // what the beams and both buffers allow a lane of 16 beams to load at a time
     const uintptr_t grid = reinterpret_cast<uintptr_t>(d_tfb) | reinterpret_cast<uintptr_t>(d_tdb) |
                            (uintptr_t)nbeams;
-    const int align = grid % 16 == 0 ? 16 : grid % 8 == 0 ? 8 : grid % 4 == 0 ? 4 : 0;
-    const bool wide = align != 0 && (size_t)nchans * sizeof(long long) <= 48 * 1024;
+    SW_REQUIRE(grid % 4 == 0, "sw_incoherent_dedisperse: the TFB and TDB must be aligned to 4 bytes");
+    const int nout = (nsamples - max_delay) / tscrunch;
+    const int align = grid % 16 == 0 ? 16 : grid % 8 == 0 ? 8 : 4;
+    // idd_k only where a CTA's table of 64-bit row offsets outgrows 48 KB of
+    // shared memory (above 6144 channels)
+    const bool wide = (size_t)nchans * sizeof(long long) <= 48 * 1024;
     const int nlanes = swb::cdiv(nbeams, wide ? 16 : 4);  // threads per (DM, sample)
     // wide: CTAs of (128 / lw) output samples x lw lanes of 16 beams
     const int lw = wide ? (nlanes < 32 ? nlanes : 32) : 128;

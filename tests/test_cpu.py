@@ -188,6 +188,19 @@ def test_c_abi_rejects_bad_arguments_without_gpu():
     assert rc == 1 and b"stages" in L.sw_last_error()
 
 
+@pytest.mark.parametrize("tfb,tdb", [(0x10001, 0x20000), (0x10000, 0x20002), (0x10003, 0x20003)])
+def test_incoherent_dedispersion_rejects_buffers_off_the_word_grid(tfb, tdb):
+    """Every form of the dedisperser reads and writes 32-bit words at least:
+    buffers off the 4-byte grid are refused on the host, before any launch."""
+    import ctypes
+
+    from skyweaver_b200 import _lib
+    L = _lib.lib()
+    rc = L.sw_incoherent_dedisperse(ctypes.c_void_p(tfb), 64, 4, 16, ctypes.c_void_p(0x30000), 2,
+                                    8, 1, 1.0, ctypes.c_void_p(tdb), None)
+    assert rc == 1 and b"aligned to 4 bytes" in L.sw_last_error()
+
+
 def test_output_description_follows_described_vector():
     """stages.describe: the DescribedVector metadata of a pipeline output
     (DescribedVector.hpp:96-573, CoherentBeamformer.cu:235,
