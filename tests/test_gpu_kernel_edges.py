@@ -228,3 +228,30 @@ def test_incoherent_dedispersion_quantiser(cuda, oracle, B, scale):
     ref = oracle.idd(tfb, delays, maxd, ts, np.float32(scale))
     got = stages.incoherent_dedisperse(_dev(cuda, tfb), _dev(cuda, delays), maxd, ts, scale)
     assert np.array_equal(_np(got), ref)
+
+
+@pytest.mark.parametrize("scale", [1.0, 3.0, 0.37, 2.9999998, -1.0, 7.0])
+def test_incoherent_dedispersion_saturated(cuda, oracle, scale):
+    """Sums on, next to and far beyond the quantiser's limits (quotients of
+    127, 128, -128, -129 and their neighbours by one unit of the sum, and all
+    128 x 11 of the largest sums) against the oracle's division."""
+    from skyweaver_b200 import stages
+    F, D, B, maxd = 11, 2, 64, 3
+    want = sorted({s for q in (126, 127, 128, 129, 200, 1397) for e in (-1, 0, 1)
+                   for s in (int(q * abs(scale)) + e, -int(q * abs(scale)) + e)
+                   if abs(s) <= 127 * F})
+    nout = -(-len(want) // B)
+    sums = np.resize(np.array(want), nout * B).reshape(nout, B)
+    tfb = np.zeros((maxd + nout, F, B), np.int64)
+    left = np.zeros((maxd + nout, B), np.int64)
+    left[maxd:] = sums
+    for f in range(F):  # spread each sum over the channels
+        tfb[:, f] = np.clip(left, -127, 127)
+        left -= tfb[:, f]
+    assert not left.any()
+    tfb = tfb.astype(np.int8)
+    delays = np.zeros((D, F), np.int32)
+    delays[1, ::2] = maxd
+    ref = oracle.idd(tfb, delays, maxd, 1, np.float32(scale))
+    got = stages.incoherent_dedisperse(_dev(cuda, tfb), _dev(cuda, delays), maxd, 1, scale)
+    assert np.array_equal(_np(got), ref)
