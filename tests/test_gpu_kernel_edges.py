@@ -255,3 +255,54 @@ def test_incoherent_dedispersion_saturated(cuda, oracle, scale):
     ref = oracle.idd(tfb, delays, maxd, 1, np.float32(scale))
     got = stages.incoherent_dedisperse(_dev(cuda, tfb), _dev(cuda, delays), maxd, 1, scale)
     assert np.array_equal(_np(got), ref)
+
+
+def _idd_rows(torch, tfb, delays, max_delay, ts, scale, lo, hi):
+    """Outputs lo .. hi - 1 in plain torch: sums in int32, one float division,
+    truncation and clamp."""
+    out = []
+    for row in delays.tolist():
+        acc = torch.zeros((hi - lo, tfb.shape[2]), dtype=torch.int32, device=tfb.device)
+        for f, d in enumerate(row):
+            s = max_delay - d + lo * ts
+            acc += tfb[s:s + (hi - lo) * ts, f].to(torch.int32).view(hi - lo, ts, -1).sum(
+                1, dtype=torch.int32)
+        out.append((acc.float() / scale).trunc().clamp(-128, 127).to(torch.int8))
+    return torch.stack(out, 1)
+
+
+@pytest.mark.parametrize("F,B", [(6144, 8), (6145, 4), (6500, 12), (6145, 16)])
+def test_incoherent_dedispersion_many_channels(cuda, F, B):
+    """On either side of the 6144 channels whose row offsets fit a CTA's
+    table: beyond, the general kernel reads them from the delays."""
+    from skyweaver_b200 import stages
+    torch = cuda
+    g = np.random.default_rng(F)
+    ts, nout, maxd = 2, 21, 15
+    delays = _dev(cuda, g.integers(0, maxd + 1, size=(3, F)).astype(np.int32))
+    delays[0, 0] = maxd
+    tfb = _dev(cuda, g.integers(-128, 128, size=(maxd + nout * ts, F, B)).astype(np.int8))
+    got = stages.incoherent_dedisperse(tfb, delays, maxd, ts, 300.0)
+    assert torch.equal(got, _idd_rows(torch, tfb, delays, maxd, ts, torch.tensor(300.0, device="cuda"), 0, nout))
+
+
+@pytest.mark.parametrize("B,gib", [(1024, 33), (1028, 9)])
+def test_incoherent_dedispersion_64_bit_offsets(cuda, B, gib):
+    """Blocks past 2^31 load units (of 16 and of 4 bytes) keep their row
+    offsets in 64 bits: delays that reach from the end of such a block to its
+    start, outputs at both ends against plain torch."""
+    from skyweaver_b200 import stages
+    torch = cuda
+    if torch.cuda.mem_get_info()[0] < (gib + 4) << 30:
+        pytest.skip("not enough free device memory")
+    F, D, ts, nout = 64, 2, 2, 40
+    T = (gib << 30) // (F * B)
+    maxd = T - nout * ts
+    assert T * F * B // (16 if B % 16 == 0 else 4) >= 1 << 31
+    tfb = torch.empty((T, F, B), dtype=torch.int8, device="cuda")
+    for lo in range(0, T, 4096):
+        tfb[lo:lo + 4096].random_(-128, 128)
+    delays = torch.linspace(0, maxd, F, device="cuda", dtype=torch.float64).round().to(torch.int32)
+    delays = torch.stack([delays, delays.flip(0)])
+    got = stages.incoherent_dedisperse(tfb, delays, maxd, ts, 8.0)
+    assert torch.equal(got, _idd_rows(torch, tfb, delays, maxd, ts, torch.tensor(8.0, device="cuda"), 0, nout))
