@@ -405,7 +405,8 @@ typedef struct sw_tuning {
     int fft_len;            /* coherent dedispersion FFT length          */
     int overlap;            /* overlap-save overlap (samples)            */
     int lag;                /* of it, trimmed at each window's end       */
-    int cb_tiles_per_item;  /* sw_cb_shape.tiles_per_item                */
+    int cb_tiles_per_item;  /* sw_cb_shape.tiles_per_item (0: its default
+                               by launch size is the fastest)            */
     float cdd_ms, cb_ms;    /* measured per gulp at the chosen settings  */
     int cb_voltage_stages;  /* sw_cb_shape.voltage_stages                */
     int cb_weight_stages;   /* sw_cb_shape.weight_stages                 */

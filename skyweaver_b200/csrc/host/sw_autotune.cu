@@ -1,10 +1,10 @@
 // Autotuner for the per-gulp chain, keyed on (nantennas, nbeams, nchans,
 // nsamples, tscrunch, DM set): times the coherent dedisperser at every FFT
-// length that fits the DM smear, and the coherent beamformer at several
-// work-item sizes (the extent of its tiles in time) and then several
-// pipeline depths (voltage and weight copies in flight) on synthetic int8
-// data of that exact shape, and caches the fastest choice per key for the
-// life of the process.
+// length that fits the DM smear, and the coherent beamformer at the work-item
+// size (the extent of its tiles in time) that a launch takes by default, at
+// several others and then at several pipeline depths (voltage and weight
+// copies in flight) on synthetic int8 data of that exact shape, and caches the
+// fastest choice per key for the life of the process.
 //
 // The reference has no autotuner (its kernel shapes are compile-time
 // constants, skyweaver_constants.hpp:28-135); it is what picks the B200
@@ -182,14 +182,15 @@ extern "C" int sw_autotune(int nantennas, int nbeams, int nchans, int nsamples, 
                                                 static_cast<int*>(map.p), stream);
         }, s, 3, ms);
     };
-    // work-item size (the tile's extent in time) at the default depths, and then
-    // the depths, starting from what a launch takes by default; another choice
-    // has to be 2 % faster, which is more than three repetitions scatter
-    // (choices within the scatter picked 128 tiles and 3 stages for the
-    // benchmark, 1-3 % behind the default in long runs)
+    // What a launch takes by default (size 0: chosen by its shape) comes first,
+    // then fixed work-item sizes (the tile's extent in time) at the default
+    // depths, then the depths at the size found.  Another choice has to be 2 %
+    // faster, which is more than three repetitions scatter (choices within the
+    // scatter picked 128 tiles and 3 stages for the benchmark, 1-3 % behind the
+    // default in long runs).
     const float kGain = 0.98f;
-    for(int tpi : {64, 4, 8, 16, 32, 128}) {
-        if(tpi > T / 64 && tpi != 4) continue;
+    for(int tpi : {0, 64, 4, 8, 16, 32, 128}) {
+        if(tpi > T / 64) continue;
         float ms = 0.0f;
         SW_TRY(time_cb(tpi, 4, 2, &ms));
         if(ms < kGain * best.cb_ms) {

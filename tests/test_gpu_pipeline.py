@@ -274,7 +274,7 @@ def test_autotune_choices_and_results(cuda, oracle):
     dms = [0.0, 150.0]
     t = stages.autotune(A, B, F, T, ts, dms, centre, bw)
     assert t["fft_len"] > t["overlap"] and t["fft_len"] & (t["fft_len"] - 1) == 0
-    assert t["cb_tiles_per_item"] in (4, 8, 16, 32, 64, 128)
+    assert t["cb_tiles_per_item"] in (0, 4, 8, 16, 32, 64, 128)  # 0: the launch's default
     assert (t["cb_voltage_stages"], t["cb_weight_stages"]) in (
         (4, 2), (2, 2), (3, 2), (6, 2), (8, 2), (4, 3), (6, 3))
     assert t["cdd_ms"] > 0 and t["cb_ms"] > 0
@@ -296,6 +296,49 @@ def test_autotune_choices_and_results(cuda, oracle):
         outs.append(pipe.outputs(0)["cb"])
         pipe.close()
     assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("A,B,F,T,ts", [(64, 128, 8, 1024, 4), (16, 64, 8, 4096, 4)])
+def test_autotuned_work_items_keep_up_with_the_default(cuda, A, B, F, T, ts):
+    """Small launches, whose default work item is shorter than the fixed sizes
+    the autotuner times (1 and 4 tiles here): its choice is the default or no
+    slower.  25 % covers the scatter of three 10 us launches; the fixed sizes
+    alone gave 1.3 to 2 times the default's time."""
+    torch = cuda
+    from skyweaver_b200 import stages
+    t = stages.autotune(A, B, F, T, ts, [0.0], 1284e6, F * 856e6 / 1024)
+    v = torch.randint(-20, 20, (F, 2, A, 2, T), dtype=torch.int8, device="cuda")
+    w = torch.randint(-127, 127, (F, 2, B, A, 2), dtype=torch.int8, device="cuda")
+    one = torch.full((F,), 1e9, device="cuda")
+    mapping = torch.zeros(B, dtype=torch.int32, device="cuda")
+    out = torch.empty((T // ts, F, B), dtype=torch.int8, device="cuda")
+
+    def launch(**how):
+        stages.coherent_beamform_grouped([(v, out, None, 0, B)], w, one, one, mapping, T, ts,
+                                         ib_subtract=False, **how)
+
+    def time_us(**how):
+        launch(**how)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(20):
+                launch(**how)
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        best = float("inf")
+        for _ in range(10):
+            e[0].record()
+            g.replay()
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]) * 50.0)
+        return best
+
+    tuned = time_us(tiles_per_item=t["cb_tiles_per_item"], voltage_stages=t["cb_voltage_stages"],
+                    weight_stages=t["cb_weight_stages"])
+    default = time_us()
+    print(t, "tuned", tuned, "default", default)
+    assert tuned <= 1.25 * default
 
 
 def test_uhf_pipeline_with_incoherent_dedispersion_vs_oracle(cuda, oracle):
