@@ -397,8 +397,8 @@ int sw_idd_pipeline_geometry(const sw_idd_pipeline* p, int block,
  * and the coherent beamformer at several work-item sizes (its tile shape in
  * time) and pipeline depths (voltage and weight copies in flight), on
  * synthetic data of this exact shape, and returns the fastest choice (cached
- * per key (nantennas, nbeams, nchans, nsamples, tscrunch, ndms, overlap) for
- * the process). The reference's launch shapes are compile-time constants
+ * per key (nantennas, nbeams, nchans, nsamples, tscrunch, ndms, DMs of 0,
+ * overlap) for the process). The reference's launch shapes are compile-time constants
  * (skyweaver_constants.hpp:28-135); this has no counterpart there. Needs a
  * few GB of device memory while it runs. */
 typedef struct sw_tuning {

@@ -9,6 +9,7 @@
 // The reference has no autotuner (its kernel shapes are compile-time
 // constants, skyweaver_constants.hpp:28-135); it is what picks the B200
 // kernels' launch shapes here.
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -43,7 +44,7 @@ struct Dev {
     }
 };
 
-using Key = std::tuple<int, int, int, int, int, int, int>;
+using Key = std::tuple<int, int, int, int, int, int, int, int>;
 std::mutex g_mu;
 std::map<Key, sw_tuning> g_cache;
 
@@ -86,7 +87,9 @@ extern "C" int sw_autotune(int nantennas, int nbeams, int nchans, int nsamples, 
     const int head    = cdd_head(centre_frequency, bandwidth, nchans, h_dms, ndms);
     const int lag     = cdd_round_lag(0, head);
     const int overlap = head + lag;
-    const Key key{nantennas, nbeams, nchans, nsamples, tscrunch, ndms, overlap};
+    // DMs of exactly 0 skip their inverse transforms, so their number counts too
+    const int nzero   = (int)std::count(h_dms, h_dms + ndms, 0.0f);
+    const Key key{nantennas, nbeams, nchans, nsamples, tscrunch, ndms, nzero, overlap};
     {
         std::lock_guard<std::mutex> lk(g_mu);
         auto it = g_cache.find(key);
