@@ -572,6 +572,7 @@ cdd_pk_kernel(const __grid_constant__ Args A)
         asm volatile("cp.async.wait_all;" ::: "memory");
         pk_sync<LOGN>(g);
         copy_zero_dms<N, NT>(stage, A, zero_dms, stream, start, L, head, copy16, t);
+        __syncwarp();  // lanes leave the copy at different lengths; see pk_sync
         Pk x[16];
 #pragma unroll
         for(int r = 0; r < 16; ++r) {

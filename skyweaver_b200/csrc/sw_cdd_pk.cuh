@@ -352,12 +352,15 @@ struct PkGroup {
 };
 
 // Barrier of one window's threads (named barriers 1 .. W; a warp for N = 1024).
+// bar.sync and the tensor memory instructions need a converged warp, and the
+// stores and copies before them leave lanes on different sides of their bounds:
+// __syncwarp joins them wherever such code ends.
 template <int LOGN>
 __device__ __forceinline__ void pk_sync(const PkGroup& g)
 {
     constexpr int T = PkGeo<LOGN>::T;
-    if constexpr(T == 32) __syncwarp();
-    else asm volatile("bar.sync %0, %1;" ::"r"(1 + g.window), "n"(T) : "memory");
+    __syncwarp();
+    if constexpr(T > 32) asm volatile("bar.sync %0, %1;" ::"r"(1 + g.window), "n"(T) : "memory");
 }
 
 __device__ __forceinline__ Pk pk_load(const uint8_t* p)
@@ -455,6 +458,7 @@ __device__ __forceinline__ void pk_forward(const PkGroup& g, Pk* x, F after_p0)
     for(int q = 0; q < 16; ++q) pk_store(g.p0 + q * G::STEP0, x[q]);
     pk_sync<LOGN>(g);
     after_p0();
+    __syncwarp();
     tm_ld16(g.tm_tw1, w[0]);
 #pragma unroll
     for(int q = 0; q < 16; ++q) x[q] = pk_load(g.p1 + G::off1(q));
