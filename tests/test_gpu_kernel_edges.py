@@ -138,6 +138,32 @@ def test_coherent_dedispersion_windows(cuda, n, F, P, A, T, ov, lag, dms, pad):
         assert float((f - ref).abs().max()) <= tol
 
 
+@pytest.mark.parametrize("n", [1024, 2048, 4096, 8192, 16384])
+@pytest.mark.parametrize("T,pad,lag", [(37, 0, 16), (5001, 7, 19), (2047, 2, 0)])
+def test_coherent_dedispersion_uneven_lanes(cuda, n, T, pad, lag):
+    """Copies of zero DMs, staging and trimmed stores that end inside a warp,
+    before its barriers and tensor memory accesses: the bytes of the same
+    samples in rows where all lanes end together, launch after launch."""
+    from skyweaver_b200 import stages
+    torch = cuda
+    ov, chbw, F, A = 208, 856e6 / 1024, 2, 37
+    dms = [0.0, 4.0, 0.0, 9.0]
+    g = np.random.default_rng(n + T)
+    T16, ov16 = -(-T // 16) * 16, ov
+    rows = np.zeros((F, 2, A, 2, ov16 + T16), np.int8)
+    rows[..., :ov + T] = np.rint(g.normal(0, 12, size=(F, 2, A, 2, ov + T)))
+    even = _dev(cuda, rows)
+    uneven = _dev(cuda, np.ascontiguousarray(rows[..., :ov + T + pad]) if ov + T + pad <= rows.shape[-1]
+                  else np.pad(rows[..., :ov + T], [(0, 0)] * 4 + [(0, pad)]))
+    cdd = stages.CoherentDedisperser(F, A, n, ov, 1257e6, F * chbw, dms, lag=lag)
+    ref = cdd.dedisperse(even, T16)
+    for _ in range(3):
+        outs = [torch.full((F, 2, A, 2, T + pad), 99, dtype=torch.int8, device="cuda") for _ in dms]
+        cdd.dedisperse(uneven, T, outs=outs)
+        for o, r in zip(outs, ref):
+            assert torch.equal(o[..., :T], r[..., :T]) and bool((o[..., T:] == 99).all())
+
+
 @pytest.mark.parametrize("A,T,ts,S,stokes,sigma", [
     (1, 16, 16, 1, "I", 8), (3, 48, 4, 1, "Q", 8), (65, 1040, 8, 9, "I", 8), (200, 544, 32, 2, "V", 8),
     (64, 528, 16, 8, "IQUV", 8), (7, 2064, 4, 3, "IQUV", 60), (64, 512, 8, 2, "I", 90),
