@@ -519,6 +519,16 @@ cdd_kernel(const __grid_constant__ Args A)
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// A chirp with a bin that is no number (a DM that is none, or a channel with a
+// bin at 0 Hz) makes every sample of its windows none, and their bytes 0: one
+// sample tells.
+__device__ __forceinline__ bool no_number(const Pk& x)
+{
+    float lo, hi;
+    unpk2(x.re, lo, hi);
+    return isnan(lo);
+}
+
 // Windows of 1024 .. 8192 points: 16384 / N windows per CTA, each by a group of
 // N / 32 threads with its own barrier and staging buffer (sw_cdd_pk.cuh).
 //
@@ -597,12 +607,21 @@ cdd_pk_kernel(const __grid_constant__ Args A)
             uint8_t* o_re = A.out[d] + out_at;
             uint8_t* o_im = o_re + A.out_stride;
             const bool words = even && (reinterpret_cast<uintptr_t>(A.out[d]) & 1) == 0;
+            const bool none = no_number(x[0]);
+            if constexpr(!DBG) {
+                if(none) {
+#pragma unroll
+                    for(int r = 0; r < 16; ++r) x[r] = {0, 0};
+                }
+            }
 #pragma unroll
             for(int r = 0; r < 16; ++r) {
                 const int u = 2 * t + (N / 16) * r - head;
                 uint32_t ra, rb, ia, ib;
                 unpk2u(pfma(x[r].re, scale, magic), ra, rb);
                 unpk2u(pfma(x[r].im, scale, magic), ia, ib);
+                if constexpr(DBG)
+                    if(none) ra = rb = ia = ib = 0;
                 if(words) {
                     if((unsigned)u < kept) {
                         *reinterpret_cast<uint16_t*>(o_re + u) =
@@ -860,6 +879,7 @@ cdd_split_combine(const __grid_constant__ SplitArgs A)
             z[k1] = {pk2(re.x, re.y), pk2(im.x, im.y)};
         }
         pdft<S, true>(z);  // z[n1] = sum_k1 W_S^(-n1 k1) z'[k1]
+        const bool none = no_number(z[0]);
         const bool words = even && !A.dbg && (reinterpret_cast<uintptr_t>(A.out[d]) & 1) == 0;
 #pragma unroll
         for(int n1 = 0; n1 < S; ++n1) {
@@ -867,6 +887,7 @@ cdd_split_combine(const __grid_constant__ SplitArgs A)
             uint32_t re[2], im[2];
             unpk2u(pfma(z[n1].re, scale, magic), re[0], re[1]);
             unpk2u(pfma(z[n1].im, scale, magic), im[0], im[1]);
+            if(none) re[0] = re[1] = im[0] = im[1] = 0;
             if(words) {
                 if((unsigned)v < kept) {
                     *reinterpret_cast<uint16_t*>(o_re + v) =
@@ -1019,11 +1040,9 @@ __global__ void chirp_k(c32* chirp, SetupArgs S)
         double sn, cs;
         sincos(phase, &sn, &cs);
         if(pk) {
-            // a chirp that is no number (a DM that is none) gives zeros
-            const bool ok = isfinite(cs) && isfinite(sn);
             float* w = reinterpret_cast<float*>(chirp + (i - q)) + b.word;
-            w[0] = ok ? (float)cs : 0.0f;
-            w[2] = ok ? (float)sn : 0.0f;
+            w[0] = (float)cs;
+            w[2] = (float)sn;
         } else {
             chirp[i] = c32{(float)cs, (float)sn};
         }
@@ -1049,10 +1068,9 @@ __global__ void chirp_split_k(c32* chirp, SetupArgs S, int split)
         const double phase = (nu * nu * S.prefactor[d]) / ((nu0 + nu) * nu0 * nu0);
         double sn, cs;
         sincos(phase, &sn, &cs);
-        const bool ok = isfinite(cs) && isfinite(sn);
         float* w = reinterpret_cast<float*>(chirp + (i - qq)) + b.word;
-        w[0] = ok ? (float)cs : 0.0f;
-        w[2] = ok ? (float)sn : 0.0f;
+        w[0] = (float)cs;
+        w[2] = (float)sn;
     }
 }
 

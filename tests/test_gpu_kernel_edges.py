@@ -164,6 +164,30 @@ def test_coherent_dedispersion_uneven_lanes(cuda, n, T, pad, lag):
             assert torch.equal(o[..., :T], r[..., :T]) and bool((o[..., T:] == 99).all())
 
 
+@pytest.mark.parametrize("n", [512, 1024, 4096, 8192, 16384])
+def test_coherent_dedispersion_without_a_number(cuda, n):
+    """A chirp with a bin that is no number (a DM that is none; in a band from
+    0 Hz the first channel's bin at 0 Hz, where the phase is a division by 0)
+    reaches every sample of that channel: no numbers in the float output, zeros
+    in the bytes, and nothing in the other channels and DMs."""
+    from skyweaver_b200 import stages
+    torch = cuda
+    F, A, T, ov = 2, 3, 900, 64
+    g = np.random.default_rng(n)
+    ext = _dev(cuda, np.rint(g.normal(0, 20, size=(F, 2, A, 2, ov + T))).astype(np.int8))
+    nan, inf = float("nan"), float("inf")
+    for low, dms, none in ((0.0, [1e-9, 2e-9], [[0], [0]]), (1257e6, [30.0, nan, inf], [[], [0, 1], [0, 1]])):
+        cdd = stages.CoherentDedisperser(F, A, n, ov, low, F * 856e6 / 1024, dms, lag=16)
+        outs, dbg = cdd.dedisperse(ext, T, debug=True)
+        plain = cdd.dedisperse(ext, T)
+        for d, channels in enumerate(none):
+            for f in range(F):
+                assert bool(torch.isnan(dbg[d, f]).all() if f in channels
+                            else torch.isfinite(dbg[d, f]).all())
+                for o in (outs, plain):
+                    assert bool((o[d][f] == 0).all()) == (f in channels)
+
+
 @pytest.mark.parametrize("A,T,ts,S,stokes,sigma", [
     (1, 16, 16, 1, "I", 8), (3, 48, 4, 1, "Q", 8), (65, 1040, 8, 9, "I", 8), (200, 544, 32, 2, "V", 8),
     (64, 528, 16, 8, "IQUV", 8), (7, 2064, 4, 3, "IQUV", 60), (64, 512, 8, 2, "I", 90),
