@@ -201,6 +201,7 @@ struct Args {
     int lag;           // trimmed at the end of each window (output delay)
     int nseg;
     int ndms;
+    int ndmg, dm_group;  // cdd_pk_kernel: DM groups of a window, DMs of a group
     const c32* tw;     // twiddle tables
     const c32* chirp;  // [ndms][F][N] in per-thread load order (chirp_k)
     size_t chirp_dm_stride;    // complex entries between two DMs' tables
@@ -529,6 +530,12 @@ __device__ __forceinline__ bool no_number(const Pk& x)
     return isnan(lo);
 }
 
+// bits d0 .. d1 - 1 of a mask of the first 32 DMs
+__device__ __forceinline__ uint32_t dm_bits(int d0, int d1)
+{
+    return (d1 < 32 ? (1u << d1) - 1u : ~0u) & ~(d0 < 32 ? (1u << d0) - 1u : ~0u);
+}
+
 // Windows of 1024 .. 8192 points: 16384 / N windows per CTA, each by a group of
 // N / 32 threads with its own barrier and staging buffer (sw_cdd_pk.cuh).
 //
@@ -541,7 +548,7 @@ __device__ __forceinline__ bool no_number(const Pk& x)
 // one DM, with 2048 points 0.285 -> 0.207 ms.  With 16 warps of 126 registers per
 // SM no unit is saturated: FMA pipe and shared-memory wavefronts 54 %, issue
 // 48 %.  (Barriers for the whole group after every pass: 5.81 ms.)
-template <int LOGN, bool DBG>
+template <int LOGN, bool DBG, bool SPLIT>
 __global__ void __launch_bounds__(kPkThreads, 1)
 cdd_pk_kernel(const __grid_constant__ Args A)
 {
@@ -550,14 +557,17 @@ cdd_pk_kernel(const __grid_constant__ Args A)
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint32_t s_tmem;
     PkGroup g;
-    const uint32_t tmem = pk_setup<LOGN>(g, smem, &s_tmem, reinterpret_cast<const float*>(A.tw));
+    const uint32_t tmem =
+        pk_setup<LOGN, true>(g, smem, &s_tmem, reinterpret_cast<const float*>(A.tw));
     const int t = g.t;
     uint8_t* stage = smem + kPkBufBytes + g.window * 2 * N;
 
     const int L = N - A.overlap;
     const int head = A.overlap - A.lag;  // trimmed at the start of each window
     const float inv_n = 1.0f / (float)N;  // exact (power of two)
-    const int nitems = A.nstreams * A.nseg;
+    // a unit of work: a window, or (SPLIT) one group of its DMs
+    const int ngroups = SPLIT ? A.ndmg : 1;
+    const int nunits = A.nstreams * A.nseg * ngroups, step = G::W * gridDim.x;
     const bool aligned = (A.row_stride % 16 == 0) && (L % 16 == 0) &&
                          ((reinterpret_cast<uintptr_t>(A.in) & 15) == 0);
     // DMs of exactly 0: copied from the staged window (see cdd_kernel)
@@ -571,17 +581,21 @@ cdd_pk_kernel(const __grid_constant__ Args A)
     // v / N rounded to the nearest even integer in the low mantissa bits (v / N
     // is below 2^14 in magnitude): the low byte is the int8-wrapped sample
     const uint64_t scale = pk2(inv_n, inv_n), magic = pk2(12582912.0f, 12582912.0f);
-    const int step = G::W * gridDim.x;
-    int item = g.window * gridDim.x + blockIdx.x;
-    if(item < nitems) stage_input<N, NT>(stage, A, item, L, aligned, t);
-    for(; item < nitems; item += step) {
+    int unit = g.window * gridDim.x + blockIdx.x;
+    if(unit < nunits) stage_input<N, NT>(stage, A, unit / ngroups, L, aligned, t);
+    for(; unit < nunits; unit += step) {
+        // window `item`, DMs d0 .. d1 - 1
+        const int item = unit / ngroups;
+        const int d0 = SPLIT ? (unit - item * ngroups) * A.dm_group : 0;
+        const int d1 = SPLIT ? min(A.ndms, d0 + A.dm_group) : A.ndms;
         const int stream = item / A.nseg;
         const int seg    = item - stream * A.nseg;
         const int f      = stream / A.npa;
         const int start  = seg * L;  // first input sample of the window
         asm volatile("cp.async.wait_all;" ::: "memory");
         pk_sync<LOGN>(g);
-        copy_zero_dms<N, NT>(stage, A, zero_dms, stream, start, L, head, copy16, t);
+        copy_zero_dms<N, NT>(stage, A, SPLIT ? zero_dms & dm_bits(d0, d1) : zero_dms, stream,
+                             start, L, head, copy16, t);
         __syncwarp();  // lanes leave the copy at different lengths; see pk_sync
         Pk x[16];
 #pragma unroll
@@ -593,15 +607,15 @@ cdd_pk_kernel(const __grid_constant__ Args A)
         }
         // the next window's bytes are fetched behind this one's transforms
         pk_forward<LOGN>(g, x, [&] {
-            if(item + step < nitems)
-                stage_input<N, NT>(stage, A, item + step, L, aligned, t);
+            if(unit + step < nunits)
+                stage_input<N, NT>(stage, A, (unit + step) / ngroups, L, aligned, t);
         });
         const float4* chp = reinterpret_cast<const float4*>(A.chirp + (size_t)f * N) + t;
         // samples of this window that the output holds: window index head + u,
         // output sample start + u, u < kept
         const unsigned kept = (unsigned)max(0, min(L, A.nsamples - start));
         const size_t out_at = (size_t)stream * 2 * A.out_stride + start;
-        for(int d = 0; d < A.ndms; ++d) {
+        for(int d = d0; d < d1; ++d) {
             if(d < 32 && ((zero_dms >> d) & 1u)) continue;
             pk_inverse<LOGN>(g, chp + (size_t)d * A.chirp_dm_stride / 2, x);
             uint8_t* o_re = A.out[d] + out_at;
@@ -723,7 +737,8 @@ cdd_split_kernel(const __grid_constant__ SplitArgs A)
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint32_t s_tmem;
     PkGroup g;
-    const uint32_t tmem = pk_setup<LOGN>(g, smem, &s_tmem, reinterpret_cast<const float*>(A.tw));
+    const uint32_t tmem =
+        pk_setup<LOGN, false>(g, smem, &s_tmem, reinterpret_cast<const float*>(A.tw));
     const int t = g.t;
     const int L = N - A.overlap;
     const int avail = A.overlap + A.nsamples;
@@ -1109,26 +1124,38 @@ int launch_logn_dbg(const Args& a, cudaStream_t stream)
     return SW_OK;
 }
 
-template <int LOGN, bool DBG>
-int launch_pk_dbg(const Args& a, cudaStream_t stream)
+template <int LOGN, bool DBG, bool SPLIT>
+int launch_pk_instance(const Args& a, long units, int nsm, cudaStream_t stream)
 {
     const size_t smem = kPkBufBytes + kPkStageBytes;
-    SW_CUDA_CHECK(cudaFuncSetAttribute(cdd_pk_kernel<LOGN, DBG>,
+    SW_CUDA_CHECK(cudaFuncSetAttribute(cdd_pk_kernel<LOGN, DBG, SPLIT>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     // the first window of every SM before the second of any
-    const long items = (long)a.nstreams * a.nseg;
-    cdd_pk_kernel<LOGN, DBG><<<(int)std::min<long>(items, nsm), kPkThreads, smem, stream>>>(a);
+    const int ctas = (int)std::min<long>(units, nsm);
+    cdd_pk_kernel<LOGN, DBG, SPLIT><<<ctas, kPkThreads, smem, stream>>>(a);
     SW_LAUNCH_CHECK();
     return SW_OK;
 }
 
 template <int LOGN>
-int launch_pk(const Args& a, cudaStream_t stream)
+int launch_pk(Args a, cudaStream_t stream)
 {
-    return a.dbg ? launch_pk_dbg<LOGN, true>(a, stream) : launch_pk_dbg<LOGN, false>(a, stream);
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const long items = (long)a.nstreams * a.nseg;
+    if(a.dbg) return launch_pk_instance<LOGN, true, false>(a, items, nsm, stream);
+    // A window's DMs are one group's serial chain, 1.9 us apiece for a lone
+    // warp of 1024 points.  Launches with fewer windows than the SMs can run
+    // side by side (groups of up to four warps, one per scheduler) share the
+    // DMs between groups, each with its own forward transform: 64 windows and 8
+    // DMs 21.7 -> 8.6 us at 1024 points, 22.9 -> 11.1 at 2048, 34.7 -> 21.7 at 8192.
+    const long groups = (long)nsm * std::max(1, 128 / PkGeo<LOGN>::T);
+    const int share = (int)std::max(1l, std::min<long>(a.ndms, groups / items));
+    if(share == 1) return launch_pk_instance<LOGN, false, false>(a, items, nsm, stream);
+    a.dm_group = cdiv(a.ndms, share);
+    a.ndmg     = cdiv(a.ndms, a.dm_group);
+    return launch_pk_instance<LOGN, false, true>(a, items * a.ndmg, nsm, stream);
 }
 
 // the float output for precision studies is a separate instance, so the

@@ -373,13 +373,53 @@ __device__ __forceinline__ void pk_store(uint8_t* p, const Pk& x)
     *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(x.re, x.im);
 }
 
+// Twiddles of thread t to tensor memory, Q quads in flight at a time.
+template <int LOGN, int Q>
+__device__ __forceinline__ void pk_fill(const float4* t0, int t, uint32_t tm)
+{
+    using G = PkGeo<LOGN>;
+#pragma unroll 1
+    for(int c = 0; c < 32; c += Q) {
+        float4 w[Q];
+#pragma unroll
+        for(int i = 0; i < Q; ++i) {
+            const int q = (c & 15) + i;
+            w[i] = q >= 15  ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)
+                   : c < 16 ? t0[q * G::T + t]
+                            : t0[G::TW0 + q * (G::R2 / 2) + t % (G::R2 / 2)];
+        }
+#pragma unroll
+        for(int i = 0; i < Q; i += 4) {
+            uint32_t v[16];
+#pragma unroll
+            for(int k = 0; k < 4; ++k) {
+                v[4 * k]     = __float_as_uint(w[i + k].x);
+                v[4 * k + 1] = __float_as_uint(w[i + k].y);
+                v[4 * k + 2] = __float_as_uint(w[i + k].z);
+                v[4 * k + 3] = __float_as_uint(w[i + k].w);
+            }
+            tm_st16(tm + (c < 16 ? 0 : 128 - 64) + 4 * (c + i), v);
+        }
+    }
+    tm_wait_st();
+}
+// All of a pass in flight (72 windows of 1024 points: 7.8 us, 4 at a time 9.0),
+// out of line so that its registers are the set-up's alone: inline the transforms
+// spill (2-4 % slower at 8192 points).  The split kernel spills around the call
+// (5 % slower), and fills 4 at a time.
+template <int LOGN>
+__device__ __noinline__ void pk_fill_fast(const float4* t0, int t, uint32_t tm)
+{
+    pk_fill<LOGN, 16>(t0, t, tm);
+}
+
 // Tensor memory of one CTA: 512 columns = spectra of the 4 warps that share a
 // lane quarter (64 columns each), then the pass 0 and pass 1 twiddles of the
 // (at most two) warps of a window that share it, common to all windows.
 // Called by all threads; the first window's threads (the first four warps
 // where a window is shorter) fill the twiddles.  Returns the base for
 // pk_tmem_free.
-template <int LOGN>
+template <int LOGN, bool FAST>
 __device__ __forceinline__ uint32_t pk_setup(PkGroup& g, uint8_t* bufs, uint32_t* s_tmem,
                                              const float* tw)
 {
@@ -406,26 +446,10 @@ __device__ __forceinline__ uint32_t pk_setup(PkGroup& g, uint8_t* bufs, uint32_t
     g.tm_spec = mine + 64 * (warp >> 2);
     g.tm_tw0  = mine + 256 + (G::T > 128 ? 64 * ((warp >> 2) & 1) : 0);
     g.tm_tw1  = g.tm_tw0 + 128;
-    if(threadIdx.x < (G::T > 128 ? G::T : 128)) {
-        const float4* t0 = reinterpret_cast<const float4*>(tw);
-        const float4* t1 = t0 + G::TW0;
-#pragma unroll 1
-        for(int c = 0; c < 8; ++c) {
-            uint32_t v[16];
-#pragma unroll
-            for(int i = 0; i < 4; ++i) {
-                const int q = 4 * (c & 3) + i;
-                const float4 w = q >= 15 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)
-                               : c < 4   ? t0[q * G::T + g.t]
-                                         : t1[q * (G::R2 / 2) + g.t % (G::R2 / 2)];
-                v[4 * i]     = __float_as_uint(w.x);
-                v[4 * i + 1] = __float_as_uint(w.y);
-                v[4 * i + 2] = __float_as_uint(w.z);
-                v[4 * i + 3] = __float_as_uint(w.w);
-            }
-            tm_st16((c < 4 ? g.tm_tw0 : g.tm_tw1) + 16 * (c & 3), v);
-        }
-        tm_wait_st();
+    if(threadIdx.x < (G::T > 128 ? G::T : 128)) {  // whole warps
+        const float4* quads = reinterpret_cast<const float4*>(tw);
+        if constexpr(FAST) pk_fill_fast<LOGN>(quads, g.t, g.tm_tw0);
+        else pk_fill<LOGN, 4>(quads, g.t, g.tm_tw0);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -164,6 +164,27 @@ def test_coherent_dedispersion_uneven_lanes(cuda, n, T, pad, lag):
             assert torch.equal(o[..., :T], r[..., :T]) and bool((o[..., T:] == 99).all())
 
 
+@pytest.mark.parametrize("n", [1024, 2048, 4096, 8192])
+@pytest.mark.parametrize("T,ndms", [(200, 8), (3000, 3), (9000, 33)])
+def test_coherent_dedispersion_splits_dms(cuda, n, T, ndms):
+    """A launch of few windows gives a window's DMs to several groups of
+    threads: the same bytes as in a launch that is too large for that, DMs of 0
+    in any place (from the 33rd on they are transformed)."""
+    from skyweaver_b200 import stages
+    torch = cuda
+    ov, lag, chbw = 224, 48, 856e6 / 1024
+    dms = [0.0 if d % 5 == 1 else 0.05 * d for d in range(ndms)]
+    g = np.random.default_rng(n + T)
+    one = _dev(cuda, np.rint(g.normal(0, 12, size=(1, 1, 2, 2, ov + T))).astype(np.int8))
+    many = one.repeat(1, 1, 400, 1, 1)
+    cdd = stages.CoherentDedisperser(1, 2, n, ov, 1257e6, chbw, dms, lag=lag)
+    small, large = cdd.dedisperse(one, T), cdd.dedisperse(many, T)
+    for d in range(ndms):
+        assert torch.equal(large[d], small[d].repeat(1, 1, 400, 1, 1)), d
+        if dms[d] == 0.0 and d < 32:
+            assert torch.equal(small[d], one[..., ov - lag:ov - lag + T])
+
+
 @pytest.mark.parametrize("n", [512, 1024, 4096, 8192, 16384])
 def test_coherent_dedispersion_without_a_number(cuda, n):
     """A chirp with a bin that is no number (a DM that is none; in a band from
