@@ -242,101 +242,171 @@ ib_k(IbArgs args, int bs0)
 // samples of 16 antennas at tscrunch 4 18 -> 5.6 us.
 constexpr int kIbWarps = 4;
 
-// The reference's float chain (t outer, a inner, float multiply and add) of
-// one output, from a table of its products (see ib_k), or sample by sample
-// when the antennas exceed the table.  First decides in 64 bits whether this
-// beamset's own sum is exact after all (`sum` holds it).  Stokes I of int8
-// samples is a whole number below 2^17, exact in float: the table takes it
-// from a byte transpose and one dp4a a sample in place of four conversions
-// and seven float operations, 240 -> 225 us per DM for 64 antennas, 64
-// channels of 65536 samples, three of them on the chain.
-template <int TS>
-__device__ __noinline__ float ib_chain(const IbArgs& args, int f, int t0, const float* w,
-                                       bool int_weights, int stokes, int sum)
+// Four samples of one antenna as words (p0.re, p0.im, p1.re, p1.im) from the
+// words of its four rows (a byte transpose).
+__device__ __forceinline__ void sample_words(const uint32_t* v, uint32_t* s)
 {
-    constexpr int L = TS < 16 ? TS : 16;  // samples per step
-    const size_t rs = args.row_stride;
-    const uint8_t* p0 = args.fpact + ((size_t)f * 2 * args.nant) * 2 * rs + args.offset + t0;
-    const uint8_t* p1 = p0 + (size_t)args.nant * 2 * rs;
-    if(int_weights) {
-        long long bound = 0;
-        for(int a = 0; a < args.nant; ++a) {
-            int e = 0;
-            for(int r = 0; r < 2; ++r)
-                for(int k = 0; k < TS; k += 4) {
-                    const int x = *reinterpret_cast<const int*>(p0 + (2 * a + r) * rs + k);
-                    const int y = *reinterpret_cast<const int*>(p1 + (2 * a + r) * rs + k);
-                    e = __dp4a(x, x, __dp4a(y, y, e));
-                }
-            bound += (long long)fabsf(w[a]) * e;
-        }
-        if(bound <= (1ll << 24)) return (float)sum;
+    const uint32_t t0 = __byte_perm(v[0], v[1], 0x5140), t1 = __byte_perm(v[2], v[3], 0x5140);
+    const uint32_t t2 = __byte_perm(v[0], v[1], 0x7362), t3 = __byte_perm(v[2], v[3], 0x7362);
+    s[0] = __byte_perm(t0, t1, 0x5410);
+    s[1] = __byte_perm(t0, t1, 0x7632);
+    s[2] = __byte_perm(t2, t3, 0x5410);
+    s[3] = __byte_perm(t2, t3, 0x7632);
+}
+
+// The Stokes parameter of one sample word: every term of the reference's float
+// formula is a whole number of at most 2^17, exact in float, so the sum is the
+// integer one.
+template <int STOKES>
+__device__ __forceinline__ int stokes_word(uint32_t s)
+{
+    const int lo = (int)(s & 0xffffu), hi = (int)(s >> 16);  // pol 0 / pol 1: (re, im, 0, 0)
+    if constexpr(STOKES == 0) return __dp4a((int)s, (int)s, 0);
+    else if constexpr(STOKES == 1) return 2 * __dp4a(lo, lo, 0) - __dp4a((int)s, (int)s, 0);
+    else if constexpr(STOKES == 2) return 2 * __dp4a(lo, hi, 0);
+    else {
+        const int x = (int)__byte_perm((uint32_t)hi, 0, 0x4401);  // (im1, re1, 0, 0)
+        return 2 * (__dp4a(lo & 0xff00, x, 0) - __dp4a(lo & 0xff, x, 0));
     }
+}
+
+// L samples of a row, in one load, as words v[.][r].
+template <int L>
+__device__ __forceinline__ void load_run(const uint8_t* p, uint32_t (*v)[4], int r)
+{
+    if constexpr(L == 16) {
+        const uint4 x = *reinterpret_cast<const uint4*>(p);
+        v[0][r] = x.x; v[1][r] = x.y; v[2][r] = x.z; v[3][r] = x.w;
+    } else if constexpr(L == 8) {
+        const uint2 x = *reinterpret_cast<const uint2*>(p);
+        v[0][r] = x.x; v[1][r] = x.y;
+    } else {
+        v[0][r] = *reinterpret_cast<const uint32_t*>(p);
+    }
+}
+
+// The four rows of antenna a from sample t on.
+template <int L>
+__device__ __forceinline__ void load_rows(const uint8_t* p0, const uint8_t* p1, size_t rs, int a,
+                                          int t, uint32_t (*v)[4])
+{
+    load_run<L>(p0 + 2 * a * rs + t, v, 0);
+    load_run<L>(p0 + (2 * a + 1) * rs + t, v, 1);
+    load_run<L>(p1 + 2 * a * rs + t, v, 2);
+    load_run<L>(p1 + (2 * a + 1) * rs + t, v, 3);
+}
+
+// The chain of one output over TS samples, L at a time: the products of L
+// samples and all antennas go to a table of rows of LDA, which is then walked
+// in order.
+template <int TS, int L, int LDA, int STOKES>
+__device__ __forceinline__ float chain_walk(const uint8_t* p0, const uint8_t* p1, size_t rs,
+                                            int nant, const float* w, float* x)
+{
     float power = 0.0f;
     for(int tc = 0; tc < TS; tc += L) {
-        if(args.nant <= kTableAnt) {
-            float x[L][kTableAnt];
 #pragma unroll 2
-            for(int a = 0; a < args.nant; ++a) {
-                uint32_t v[4][L / 4];
+        for(int a = 0; a < nant; ++a) {
+            uint32_t v[L / 4][4];
+            load_rows<L>(p0, p1, rs, a, tc, v);
 #pragma unroll
-                for(int k = 0; k < L / 4; ++k) {
-                    v[0][k] = *reinterpret_cast<const uint32_t*>(p0 + 2 * a * rs + tc + 4 * k);
-                    v[1][k] = *reinterpret_cast<const uint32_t*>(p0 + (2 * a + 1) * rs + tc + 4 * k);
-                    v[2][k] = *reinterpret_cast<const uint32_t*>(p1 + 2 * a * rs + tc + 4 * k);
-                    v[3][k] = *reinterpret_cast<const uint32_t*>(p1 + (2 * a + 1) * rs + tc + 4 * k);
-                }
-                if(stokes == 0) {
-                    // Stokes I of int8 voltages is a whole number below 2^17, so
-                    // the reference's float steps are exact: the four bytes of a
-                    // sample (PRMT transpose) summed as squares by one dp4a
+            for(int k = 0; k < L / 4; ++k) {
+                uint32_t s[4];
+                sample_words(v[k], s);
 #pragma unroll
-                    for(int k = 0; k < L / 4; ++k) {
-                        const uint32_t t0 = __byte_perm(v[0][k], v[1][k], 0x5140);
-                        const uint32_t t1 = __byte_perm(v[2][k], v[3][k], 0x5140);
-                        const uint32_t t2 = __byte_perm(v[0][k], v[1][k], 0x7362);
-                        const uint32_t t3 = __byte_perm(v[2][k], v[3][k], 0x7362);
-                        const uint32_t s[4] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632),
-                                               __byte_perm(t2, t3, 0x5410), __byte_perm(t2, t3, 0x7632)};
-#pragma unroll
-                        for(int i = 0; i < 4; ++i)
-                            x[4 * k + i][a] = fmul((float)__dp4a((int)s[i], (int)s[i], 0), w[a]);
-                    }
-                } else {
-#pragma unroll
-                    for(int k = 0; k < L; ++k) {
-                        auto byte = [&](int r) { return (float)(int8_t)(v[r][k / 4] >> (8 * (k & 3))); };
-                        x[k][a] = fmul(stokes_f(stokes, byte(0), byte(1), byte(2), byte(3)), w[a]);
-                    }
-                }
+                for(int i = 0; i < 4; ++i)
+                    x[(4 * k + i) * LDA + a] = fmul((float)stokes_word<STOKES>(s[i]), w[a]);
             }
-            for(int k = 0; k < L; ++k)
-                for(int a = 0; a < args.nant; ++a) power = fadd(power, x[k][a]);
-        } else {
-            for(int k = tc; k < tc + L; ++k)
-                for(int a = 0; a < args.nant; ++a)
-                    power = fadd(power, fmul(stokes_f(stokes, (float)(int8_t)p0[2 * a * rs + k],
-                                                      (float)(int8_t)p0[(2 * a + 1) * rs + k],
-                                                      (float)(int8_t)p1[2 * a * rs + k],
-                                                      (float)(int8_t)p1[(2 * a + 1) * rs + k]),
-                                             w[a]));
+        }
+        for(int k = 0; k < L; ++k) {  // 16 entries in flight
+            const float* y = x + k * LDA;
+            int a = 0;
+            for(; a + 16 <= nant; a += 16) {
+                float v[16];
+#pragma unroll
+                for(int i = 0; i < 16; ++i) v[i] = y[a + i];
+#pragma unroll
+                for(int i = 0; i < 16; ++i) power = fadd(power, v[i]);
+            }
+            for(; a < nant; ++a) power = fadd(power, y[a]);
         }
     }
     return power;
 }
 
+template <int TS, int L, int LDA>
+__device__ __forceinline__ float chain_stokes(int stokes, const uint8_t* p0, const uint8_t* p1,
+                                              size_t rs, int nant, const float* w, float* x)
+{
+    switch(stokes) {
+    case 0: return chain_walk<TS, L, LDA, 0>(p0, p1, rs, nant, w, x);
+    case 1: return chain_walk<TS, L, LDA, 1>(p0, p1, rs, nant, w, x);
+    case 2: return chain_walk<TS, L, LDA, 2>(p0, p1, rs, nant, w, x);
+    default: return chain_walk<TS, L, LDA, 3>(p0, p1, rs, nant, w, x);
+    }
+}
+
+// The reference's float chain (t outer, a inner, float multiply and add) of
+// one output, from a table of its products in local memory (see ib_k): 16
+// samples of up to kTableAnt antennas, 4 samples of more.  Where several
+// beamsets share the bound (`recheck`), first decides in 64 bits whether this
+// beamset's own sum is exact after all (`sum` holds it).
+// Whole products on sample words and a compile-time Stokes parameter take the
+// place of four conversions and up to seven float operations a product, one
+// load a row the place of four, and 16 table entries are in flight: 64 antennas
+// x 16 channels x 8192 samples at tscrunch 16 with fractional weights 52 -> 41 us
+// for I, 83 -> 42 us for Q and, with the components on four warps, 323 -> 92 us
+// for IQUV; two beamsets of I over 100 antennas, which were walked sample by
+// sample, 400 -> 149 us.  On 64 channels x 65536 samples, where the tables live
+// in L2, 853 -> 822 us for I and 2.87 -> 2.07 ms for IQUV.
+template <int TS>
+__device__ __noinline__ float ib_chain(const IbArgs& args, int f, int t0, const float* w,
+                                       bool recheck, int stokes, int sum)
+{
+    constexpr int L = TS < 16 ? TS : 16;
+    const size_t rs = args.row_stride;
+    const uint8_t* p0 = args.fpact + ((size_t)f * 2 * args.nant) * 2 * rs + args.offset + t0;
+    const uint8_t* p1 = p0 + (size_t)args.nant * 2 * rs;
+    if(recheck) {
+        long long bound = 0;
+        for(int a = 0; a < args.nant; ++a) {
+            int e = 0;
+            for(int k = 0; k < TS; k += L) {
+                uint32_t v[L / 4][4];
+                load_rows<L>(p0, p1, rs, a, k, v);
+#pragma unroll
+                for(int i = 0; i < L; ++i) {
+                    const int x = (int)v[i / 4][i & 3];
+                    e = __dp4a(x, x, e);
+                }
+            }
+            bound += (long long)fabsf(w[a]) * e;
+        }
+        if(bound <= (1ll << 24)) return (float)sum;
+    }
+    static_assert(4 * kMaxAnt == 16 * kTableAnt, "one table serves both forms");
+    float x[16 * kTableAnt];
+    if(args.nant <= kTableAnt)
+        return chain_stokes<TS, L, kTableAnt>(stokes, p0, p1, rs, args.nant, w, x);
+    return chain_stokes<TS, 4, kMaxAnt>(stokes, p0, p1, rs, args.nant, w, x);
+}
+
 // NC components (4: I, Q, U, V), NBS beamsets per pass; I_ONLY: NC = 1 and
-// Stokes I.
+// Stokes I.  Up to tscrunch 16 the bounds name one CTA per SM: without that
+// the compiler holds a kernel that calls the chain to few registers, and its
+// row loads to fewer in flight (64 channels x 65536 samples, Stokes I: one
+// beamset at tscrunch 16 159 -> 149 us, eight at 8 206 -> 182 us); at 32 its own
+// choice is 5-10 % ahead on half that many channels.
 template <int TS, int NC, int NBS, bool I_ONLY>
-__global__ void __launch_bounds__(32 * kIbWarps)
+__global__ void __launch_bounds__(32 * kIbWarps, TS < 32 ? 1 : 0)
 ib_run_k(const __grid_constant__ IbArgs args, int bs0)
 {
     constexpr int NO = TS < 16 ? 16 / TS : 1;   // outputs per thread
     constexpr int RUN = TS < 16 ? 16 : TS;      // samples per thread
     constexpr int NV = NO * (NBS * NC + 1);     // sums per thread, the bounds last
     __shared__ float sw[NBS][kMaxAnt];
-    __shared__ int s_max[kMaxAnt];              // max |w| over the beamsets, >= 2^24: not whole
-    __shared__ int s_int[NBS];
+    __shared__ int s_max[kMaxAnt];              // max |w| over the beamsets of whole weights
+    __shared__ int s_int[NBS];                  // whole weights of at most 1024
     __shared__ uint32_t red[kIbWarps][NV][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nbs = min(NBS, args.nbeamsets - bs0);
@@ -434,30 +504,30 @@ ib_run_k(const __grid_constant__ IbArgs args, int bs0)
         red[warp][NO * NBS * NC + o][lane] = B[o];
     }
     __syncthreads();
-    if(t0 >= args.nsamples) return;
-
+    // A warp per (32 consecutive outputs, component, beamset), as each may have
+    // to walk the chain: neighbouring lanes then read neighbouring samples.
     const int nout = args.nsamples / TS;
-    for(int i = warp; i < NO * nbs; i += kIbWarps) {
-        const int o = i % NO, s = i / NO, bs = bs0 + s;
-        const int tp = t0 / TS + o;
+    for(int i = warp; i < NO * NC * nbs; i += kIbWarps) {
+        const int q = i % NO * 32 + lane, c = i / NO % NC, s = i / (NO * NC), bs = bs0 + s;
+        const int o = q % NO, run = q / NO;
+        const int tp = blockIdx.x * 32 * NO + q;
+        if(tp >= nout) continue;
         uint32_t bound = 0;
-        for(int k = 0; k < kIbWarps; ++k) bound += red[k][NO * NBS * NC + o][lane];
+        for(int k = 0; k < kIbWarps; ++k) bound += red[k][NO * NBS * NC + o][run];
         const size_t at = ((size_t)bs * nout + tp) * args.nchans + f;
         const size_t so = (size_t)bs * args.nchans + f;
-        for(int c = 0; c < NC; ++c) {
-            const int stokes = NC == 4 ? c : args.stokes;
-            uint32_t sum = 0;
-            for(int k = 0; k < kIbWarps; ++k) sum += red[k][(o * NBS + s) * NC + c][lane];
-            const float power = s_int[s] && bound <= (1u << 24)
-                                    ? (float)(int)sum  // the float chain is exact
-                                    : ib_chain<TS>(args, f, tp * TS, sw[s], s_int[s] != 0, stokes,
-                                                   (int)sum);
-            args.raw[at * NC + c] = power;
-            const float sc = stokes == 0
-                                 ? rintf(fdiv(fsub(power, args.offset_v[so]), args.scale[so]))
-                                 : rintf(fdiv(power, args.scale[so]));
-            args.out[at * NC + c] = clamp_i8(sc);
-        }
+        const int stokes = NC == 4 ? c : args.stokes;
+        uint32_t sum = 0;
+        for(int k = 0; k < kIbWarps; ++k) sum += red[k][(o * NBS + s) * NC + c][run];
+        const float power = s_int[s] && bound <= (1u << 24)
+                                ? (float)(int)sum  // the float chain is exact
+                                : ib_chain<TS>(args, f, tp * TS, sw[s], s_int[s] && nbs > 1,
+                                               stokes, (int)sum);
+        args.raw[at * NC + c] = power;
+        const float sc = stokes == 0
+                             ? rintf(fdiv(fsub(power, args.offset_v[so]), args.scale[so]))
+                             : rintf(fdiv(power, args.scale[so]));
+        args.out[at * NC + c] = clamp_i8(sc);
     }
 }
 

@@ -212,7 +212,8 @@ def test_coherent_dedispersion_without_a_number(cuda, n):
 @pytest.mark.parametrize("A,T,ts,S,stokes,sigma", [
     (1, 16, 16, 1, "I", 8), (3, 48, 4, 1, "Q", 8), (65, 1040, 8, 9, "I", 8), (200, 544, 32, 2, "V", 8),
     (64, 528, 16, 8, "IQUV", 8), (7, 2064, 4, 3, "IQUV", 60), (64, 512, 8, 2, "I", 90),
-    (70, 64, 32, 1, "U", 90), (16, 32, 4, 5, "I", 127)])
+    (70, 64, 32, 1, "U", 90), (16, 32, 4, 5, "I", 127), (100, 2064, 4, 2, "IQUV", 60),
+    (65, 1040, 8, 1, "Q", 60), (256, 80, 16, 1, "I", 40), (128, 32, 32, 2, "V", 90)])
 @pytest.mark.parametrize("weights", ["masks", "large", "fractional"])
 def test_incoherent_beam_runs(cuda, oracle, A, T, ts, S, stokes, sigma, weights):
     """The 16-sample-run form against the oracle and against the general form
