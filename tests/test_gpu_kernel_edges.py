@@ -31,6 +31,27 @@ def test_layout_converters_ragged(cuda, nant, T, stride, off):
     assert np.array_equal(_np(stages.fpact_to_ftpa(fp, T, offset=off)), ftpa)
 
 
+@pytest.mark.parametrize("F,nant,T,stride,off", [
+    (1, 1, 40000, 40004, 4), (5, 2, 5003, 5003, 0), (2, 6, 4096, 4112, 13),  # a thread per antenna
+    (40, 7, 5, 8, 0), (80, 7, 250, 256, 3),          # past that: tiles
+    (23, 64, 128, 128, 0), (24, 64, 128, 128, 0),    # on either side of the tile counts that
+    (147, 64, 128, 131, 1), (148, 64, 128, 131, 1),  # part them, rows on and off the 4-byte grid
+    (160, 64, 131, 144, 13), (75, 65, 130, 132, 0), (40, 250, 129, 131, 1)])
+def test_layout_converters_forms(cuda, F, nant, T, stride, off):
+    """Both forms of the FTPA <-> FPACT converters at the lines between them,
+    whole and ragged tiles, rows on and off the 4-byte grid: equal to the
+    permutation, and the bytes outside [off, off + T) stay."""
+    from skyweaver_b200 import stages
+    torch = cuda
+    gen = torch.Generator(device="cuda").manual_seed(F + nant)
+    ftpa = torch.randint(-128, 128, (F, T, 2, nant, 2), dtype=torch.int8, device="cuda", generator=gen)
+    fp = stages.ftpa_to_fpact(ftpa, row_stride=stride, offset=off)
+    ref = torch.zeros((F, 2, nant, 2, stride), dtype=torch.int8, device="cuda")
+    ref[..., off:off + T] = ftpa.permute(0, 2, 3, 4, 1)
+    assert torch.equal(fp, ref)
+    assert torch.equal(stages.fpact_to_ftpa(fp, T, offset=off), ftpa)
+
+
 @pytest.mark.parametrize("ts,stokes", [(1, "I"), (4, "Q"), (16, "I"), (2, "IQUV"), (32, "V")])
 @pytest.mark.parametrize("ib_sub", [True, False])
 def test_coherent_beam_quantiser(cuda, oracle, ts, stokes, ib_sub):
@@ -250,6 +271,21 @@ def test_transpose_statistics_splits(cuda, H, A_in, A, F):
     ref = stages.transpose_fpact(taftp, A)
     assert bool((fp == ref).all())
     assert np.array_equal(_np(st), _np(stages.statistics(ref, H * 256)), equal_nan=True)
+
+
+@pytest.mark.parametrize("H,A_in,A,F", [(2048, 1, 8, 1), (3, 24, 24, 683), (2, 24, 24, 1023),
+                                        (3, 25, 32, 683), (2, 255, 256, 3)])
+def test_transpose_ftpa_parts(cuda, H, A_in, A, F):
+    """Whole and half heaps per CTA on either side of the antenna and CTA
+    counts that part them, antennas absent and the most there can be."""
+    from skyweaver_b200 import stages
+    torch = cuda
+    gen = torch.Generator(device="cuda").manual_seed(H + A)
+    taftp = torch.randint(-128, 128, (H, A_in, F, 256, 2, 2), dtype=torch.int8, device="cuda",
+                          generator=gen)
+    ref = torch.zeros((F, H, 256, 2, A, 2), dtype=torch.int8, device="cuda")
+    ref[:, :, :, :, :A_in] = taftp.permute(2, 0, 3, 4, 1, 5)
+    assert torch.equal(stages.transpose_ftpa(taftp, A), ref.view(F, H * 256, 2, A, 2))
 
 
 @pytest.mark.parametrize("scale,rate,age", [(1e-6, 0.0, 0.0), (3e-5, 1e-9, 3600.0), (20.0, 0.0, 0.0)])
