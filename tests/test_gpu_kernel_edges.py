@@ -82,6 +82,29 @@ def test_coherent_beam_quantiser(cuda, oracle, ts, stokes, ib_sub):
     assert np.array_equal(_np(out), ref)
 
 
+@pytest.mark.parametrize("ts,stokes", [(1, "I"), (2, "Q"), (4, "I"), (8, "U"), (8, "IQUV"),
+                                       (16, "IQUV"), (16, "I"), (32, "I")])
+def test_coherent_beam_lanes_part(cuda, oracle, ts, stokes):
+    """Beamsets that alternate from lane to lane, some of whose outputs are all
+    divided, some never, and beams missing from the last warps: every column
+    group after them is loaded by the whole warp (bit-exact)."""
+    from skyweaver_b200 import stages
+    g = np.random.default_rng(ts)
+    A, B, T, F, S = 16, 45, 1024, 3, 4
+    ftpa = g.integers(-2, 3, size=(F, T, 2, A, 2), dtype=np.int8)
+    w = g.integers(-1, 2, size=(F, B, A, 2), dtype=np.int8)
+    bw = np.ones((S, A), np.float32)
+    scl = np.repeat(np.array([2.0, 1e-35, 48.0, 7.0], np.float32), F)
+    off = np.full(S * F, 100.0, np.float32)
+    mapping = (np.arange(B) % S).astype(np.int32)
+    ref = oracle.coherent_beam(ftpa, w, ts, scl, off, bw, mapping, stokes, False)
+    out = stages.coherent_beamform(stages.ftpa_to_fpact(_dev(cuda, ftpa)),
+                                   stages.pack_weights(_dev(cuda, w)), _dev(cuda, scl),
+                                   _dev(cuda, off), _dev(cuda, mapping), None, T, ts,
+                                   stokes=stokes, ib_subtract=False)
+    assert np.array_equal(_np(out), ref)
+
+
 @pytest.mark.parametrize("B,F,T", [(1, 1, 64), (129, 2, 64), (64, 8, 4096), (300, 5, 1216),
                                    (128, 149, 128), (257, 37, 8256)])
 def test_coherent_beam_default_work_items(cuda, B, F, T):
