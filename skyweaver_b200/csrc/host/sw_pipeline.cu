@@ -15,9 +15,10 @@
 // transform and no copy.
 //
 // all ordered on one stream (the weights on a side stream forked from it and
-// joined to it), captured once as a CUDA graph per input/output buffer pair.  process_host double-buffers the pinned-host input and the outputs
-// so that the H2D of gulp g+1 and the D2H of gulp g-1 overlap the compute
-// of gulp g on separate copy streams.
+// joined to it), captured once as a CUDA graph per input/output buffer pair.
+// process_host double-buffers the pinned-host input and the outputs so that the
+// H2D of gulp g+1 and the D2H of gulp g-1 overlap the compute of gulp g on
+// separate copy streams.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -293,8 +294,10 @@ int sw_pipeline::enqueue_chain(const void* d_in, int parity, bool first)
     SW_TRY(sw_transpose_fpact_statistics(d_in, rows, nheaps, cfg.input_nantennas, A, F,
                                          ext_stride, ext_off, stats_scratch.p,
                                          stats[parity].as<float>(), ss));
-    // The channel order only matters when the incoherent beam's CTAs (32 runs
-    // of 16 samples of one channel) do not all start at once.
+    // The channel order only matters when the incoherent beam's CTAs do not
+    // start at about the same time.  4 or 5 of them fit an SM, and at tscrunch 4
+    // to 16 one takes 32 runs of 16 samples of a channel: from two rounds on the
+    // ranking (a launch of 3 to 11 us) can pay, below it cannot.
     const int* chan_order = nullptr;
     if(ib_order.p && (long)F * swb::cdiv(T, 512) > 8 * 148) {
         SW_TRY(swb::launch_ib_channel_order(stats[parity].as<float>(), F, 2, A,

@@ -13,7 +13,8 @@
 // 8192-point sub-transforms (cdd_split_kernel):
 //   * the forward FFT is in place, decimation in frequency, its first pass read
 //     straight from the staged planar int8 rows, its last pass leaving each
-//     thread's spectral bins in registers in digit-reversed order;
+//     thread's spectral bins in digit-reversed order, in registers (256 and 512
+//     points) or in tensor memory (longer windows);
 //   * for every coherent DM the thread multiplies its bins by the chirp (FP64
 //     phases, stored as complex float in the order the threads load it), runs
 //     the exact inverse passes (decimation in time, conjugate twiddles), and
@@ -545,7 +546,7 @@ __device__ __forceinline__ uint32_t dm_bits(int d0, int d1)
 // 64 antennas x 64 channels x 65536 samples at DMs 50, 150 and 500 took 9.21 ms
 // that way with 8192 points and take 5.48 ms here; 32 channels x 32768 samples
 // with 4096 points 2.10 -> 1.33 ms; 48 antennas x 32 channels x 16384 samples,
-// one DM, with 2048 points 0.285 -> 0.207 ms.  With 16 warps of 126 registers per
+// one DM, with 2048 points 0.285 -> 0.204 ms.  With 16 warps of 126 registers per
 // SM no unit is saturated: FMA pipe and shared-memory wavefronts 54 %, issue
 // 48 %.  (Barriers for the whole group after every pass: 5.81 ms.)
 template <int LOGN, bool DBG, bool SPLIT>
@@ -682,9 +683,10 @@ cdd_pk_kernel(const __grid_constant__ Args A)
 // partial DFT straight from the int8 rows into pass 0's registers, the M-point
 // forward FFT, and for every DM the chirp of bins k1 + S k2 and the M-point
 // inverse FFT (sw_cdd_pk.cuh), leaving W_N^(-n2 k1) * z in a workspace of pairs
-// (8-byte accesses: the caller's workspace need not be aligned further); cdd_split_combine then does the S-point inverse DFT over k1,
-// the overlap-save trim, /N, rint and int8 wrap.  DMs of exactly 0 are copied
-// from the rows by the combine step.
+// (8-byte accesses: the caller's workspace need not be aligned further);
+// cdd_split_combine then does the S-point inverse DFT over k1, the overlap-save
+// trim, /N, rint and int8 wrap.  DMs of exactly 0 are copied from the rows by
+// the combine step.
 // 64 antennas x 8 channels x 65536 samples at 65536 points and DMs 0, 50, 150
 // and 500: 7.46 ms with 16 points a thread in scalar arithmetic, 4.12 ms with
 // these sub-transforms, 2.72 ms with the rows loaded without a branch between

@@ -12,9 +12,11 @@
 // reference order (slow path) for outputs that fail it.  The result is
 // bit-identical to the reference's CPU implementation in both cases.
 //
-// One thread per (channel, output sample); the planar FPACT rows make each
-// thread's tscrunch samples a contiguous 4/8/16-byte load, coalesced across
-// the warp.  The kernel is HBM bound (one read of the voltages).
+// ib_k: one thread per (channel, output sample); the planar FPACT rows make
+// each thread's tscrunch samples a contiguous 4/8/16-byte load, coalesced across
+// the warp.  ib_run_k, for tscrunch 4 to 32 on aligned rows: 16-byte runs of
+// every row, the antennas over four warps.  Both are HBM bound (one read of the
+// voltages).
 #include "sw_common.cuh"
 
 namespace swb {

@@ -97,21 +97,22 @@ stats_partial_k(const uint8_t* __restrict__ fpact, size_t row_stride,
 // and add one warp-reduced set of sums per (antenna, pol) into the int64
 // workspace (the two warps of an antenna both add).  Padded antennas (a >=
 // in_nant) are written as zeros and summed as zeros, like the separate
-// stages.  The sums cost more issue than the copy, so the kernel is
-// issue-bound: on a 64 ant x 64 ch x 65536-sample gulp (with its memset) 16,
-// 8, 4, 2 and 1 heaps per CTA took 0.542, 0.498, 0.526, 0.633 and 1.042 ms,
-// against 0.342 + 0.278 ms for the separate transpose and statistics (16
-// heaps leave a second wave of CTAs that fills a third of the SMs).
-//
-// Shorter gulps give the antenna groups to gridDim.z CTAs, and then fewer heaps
-// to each, until there are kFuseCtas of them (8 CTAs of 256 threads fill an
-// SM): 57 of 64 antennas x 64 channels x 67 heaps 154 -> 140 us, 16 antennas x
-// 8 channels x 16 heaps 24 -> 6 us.
+// stages.  The sums cost more issue than the copy: 78 % of the issue slots and
+// 59 % of the ALU pipe are taken, 56 % of the HBM rate.
 //
 // The loads of kFuseBatch heaps are issued before the first is used; one at a
 // time, with the stores and sums of the one before between them, their latency
-// bound the kernel (7 of 8.5 warps per issue waited for them): batches of 1, 2,
-// 4 and 8 heaps take 496, 477, 433 and 394 us on the gulp above (5.4 TB/s).
+// bound the kernel (7 of 8.5 warps per issue waited for them): batches of 1, 4
+// and 8 heaps take 495, 430 and 389 us on a 64 antenna x 64 channel x 65536
+// sample gulp (5.5 TB/s; the separate transpose and statistics 342 + 278 us).
+// The batch takes 64 registers, so 4 CTAs fill an SM.  16, 8, 4 and 2 heaps per
+// CTA take 372, 389, 485 and 699 us there.
+//
+// Shorter gulps give the antenna groups to gridDim.z CTAs, and then fewer heaps
+// to each, until there are kFuseCtas of them.  That is two rounds of the 4
+// resident CTAs: 64 antennas x 64 channels x 16 heaps take 36.4, 38.5, 34.4,
+// 32.2 and 32.0 us with 3, 4, 5, 8 and 12 CTAs per SM asked for, 16 antennas x 16
+// channels x 32 heaps 8.9, 9.0, 9.8, 11.2 and 11.2 us (22.6 us unsplit).
 constexpr int kFuseHeaps = 8;
 constexpr int kFuseBatch = 8;
 constexpr int kFuseCtas  = 8 * 148;
