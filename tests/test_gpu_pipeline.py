@@ -343,13 +343,14 @@ def test_autotuned_work_items_keep_up_with_the_default(cuda, A, B, F, T, ts):
 
 def test_autotune_counts_the_zero_dms(cuda):
     """A DM of exactly 0 skips its inverse transform: DM sets of equal size and
-    overlap with and without it are tuned apart."""
+    overlap with and without it are tuned apart.  One of three transforms less
+    on 3000 windows shows far above the timing's scatter."""
     from skyweaver_b200 import stages
-    shape = (16, 32, 2, 4096, 16)
-    a = stages.autotune(*shape, [150.0, 150.0], 1284e6, 2 * 856e6 / 1024)
-    b = stages.autotune(*shape, [0.0, 150.0], 1284e6, 2 * 856e6 / 1024)
+    shape = (64, 32, 8, 16384, 16)
+    a = stages.autotune(*shape, [150.0, 150.0], 1284e6, 8 * 856e6 / 1024)
+    b = stages.autotune(*shape, [0.0, 150.0], 1284e6, 8 * 856e6 / 1024)
     assert a["overlap"] == b["overlap"]
-    assert (a["cdd_ms"], a["cb_ms"]) != (b["cdd_ms"], b["cb_ms"])  # measured twice, not shared
+    assert b["cdd_ms"] < 0.92 * a["cdd_ms"], (a, b)
 
 
 def test_uhf_pipeline_with_incoherent_dedispersion_vs_oracle(cuda, oracle):
